@@ -390,9 +390,9 @@ hf_status hf_repair_roundoff(hf_ctx* ctx, int nlev, const hf_level* levels, cons
     return HF_OK;
 }
 
-hf_status hf_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch, const double* U_in,
-                         const double* U_old, double* U_out, double* fx, double* fy, double h, int first_order,
-                         int form, int64_t* bad_cell, void* stream) {
+static hf_status flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch,
+                             const double* U_in, const double* U_old, double* U_out, double* fx, double* fy, double h,
+                             int first_order, int form, int64_t* bad_cell, void* stream, bool record) {
     if (bad_cell) *bad_cell = -1;
     if (!ctx || !level || !patches || npatch <= 0 || !U_in || !U_out || U_in == U_out || !level_ok(*level) ||
         !(h > 0) || (form != HF_FLUX_PLAIN && form != HF_FLUX_FUSED))
@@ -432,7 +432,7 @@ hf_status hf_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* pat
                                       &ctx->cnt.kernel_launches));
         } else if (npatch == 1) {
             HF_CUDA(launch_flux_plain(ctx->ns, L, patches[0], 0, U_in, uold, U_out, FX, FY, h, first_order, 0, ctx->st,
-                                      s, &ctx->cnt.kernel_launches));
+                                      s, &ctx->cnt.kernel_launches, nullptr, record));
         } else {
             // every patch in one launch per kernel: face arrays packed per patch in patch order
             std::vector<int64_t> off(3 * (size_t)npatch);
@@ -487,6 +487,13 @@ hf_status hf_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* pat
     }
     if (f & ST_COMBINE_BAD) return fail(ctx, HF_ERR_COMBINE, "flux_update: inadmissible Heun combination");
     return HF_OK;
+}
+
+hf_status hf_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch, const double* U_in,
+                         const double* U_old, double* U_out, double* fx, double* fy, double h, int first_order,
+                         int form, int64_t* bad_cell, void* stream) {
+    return flux_update(ctx, level, patches, npatch, U_in, U_old, U_out, fx, fy, h, first_order, form, bad_cell, stream,
+                       false);
 }
 
 hf_status hf_flux_adjoint(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U,
@@ -683,8 +690,8 @@ hf_status hf_chem_adjoint(hf_ctx* ctx, const double* U0, int64_t comp_stride, in
                             stream, true);
 }
 
-hf_status hf_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch, const double* U, double cfl,
-                    double* dt, void* stream) {
+static hf_status cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch, const double* U,
+                        double cfl, double* dt, void* stream, bool record) {
     if (!ctx || !level || !patches || npatch <= 0 || !U || !dt || !(cfl > 0) || !level_ok(*level))
         return fail(ctx, HF_ERR_ARG, "cfl_dt: bad arguments");
     for (int p = 0; p < npatch; ++p)
@@ -705,7 +712,7 @@ hf_status hf_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patches,
     HF_CUDA(reset_status(ctx, s));
     tic(ctx, 2, s);
     if (npatch == 1)
-        HF_CUDA(launch_cfl(ctx->ns, L, patches[0], U, ctx->st, s, &ctx->cnt.kernel_launches));
+        HF_CUDA(launch_cfl(ctx->ns, L, patches[0], U, ctx->st, s, &ctx->cnt.kernel_launches, record));
     else
         HF_CUDA(launch_cfl_multi(ctx->ns, L, patches, ctx->d_patches, npatch, ctx->d_off, U, ctx->st, s,
                                  &ctx->cnt.kernel_launches));
@@ -716,6 +723,11 @@ hf_status hf_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patches,
     memcpy(&rate, &ctx->st_host->rate_bits, sizeof rate);
     *dt = cfl / rate;
     return HF_OK;
+}
+
+hf_status hf_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch, const double* U, double cfl,
+                    double* dt, void* stream) {
+    return cfl_dt(ctx, level, patches, npatch, U, cfl, dt, stream, false);
 }
 
 hf_status hf_validate(hf_ctx* ctx, const hf_level* level, const hf_patch* patches, int npatch, const double* U,
@@ -925,3 +937,16 @@ hf_status hf_fp64_peak(hf_ctx* ctx, double* gflops, void* stream) {
 }
 
 }  // extern "C"
+
+namespace hf {
+hf_status record_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U_in,
+                             const double* U_old, double* U_out, double h, int first_order, void* stream) {
+    int64_t bad = -1;
+    return flux_update(ctx, level, patch, 1, U_in, U_old, U_out, nullptr, nullptr, h, first_order, HF_FLUX_PLAIN, &bad,
+                       stream, true);
+}
+hf_status record_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U, double cfl,
+                        double* dt, void* stream) {
+    return cfl_dt(ctx, level, patch, 1, U, cfl, dt, stream, true);
+}
+}  // namespace hf

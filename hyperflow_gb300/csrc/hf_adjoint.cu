@@ -317,7 +317,7 @@ __device__ __noinline__ bool chem_vjp(double rho, double e, double& T, const dou
     double z[NS], C[NS], m[6];
     comp<NS>(y, rho, z, C);
     double Tn = T;
-    if (!solve_T<NS>(z, e, Tn, m)) return false;
+    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
     T = Tn;
     KinCtx<NS> kc;
     kin_setup<NS, false>(T, C, kc);
@@ -413,7 +413,7 @@ __device__ __noinline__ bool chem_hess(double rho, double e, double& T, const do
     double z[NS], C[NS], m[6];
     comp<NS>(y, rho, z, C);
     double Tn = T;
-    if (!solve_T<NS>(z, e, Tn, m)) return false;
+    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
     T = Tn;
     KinCtx<NS> kc;
     kin_setup<NS, false>(T, C, kc);
@@ -607,7 +607,7 @@ __device__ bool state_grads(const double* u, double* dT, double* dp, double& T) 
 #pragma unroll
     for (int k = 0; k < N; ++k) y[k] = u[k] * ir;
     comp<NS>(y, rho, z, C);
-    if (!solve_T<NS>(z, e, T, m)) return false;
+    if (!solve_T_iter<NS>(z, e, T, m)) return false;
     KinCtx<NS> kc;
     kin_setup<NS, false>(T, C, kc);
     double cpR[NS], dcpR[NS], cvk[NS], cv, ETT;

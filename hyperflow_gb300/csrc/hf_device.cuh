@@ -7,13 +7,13 @@
 // The EOS closure restates what physics.cpp:4-15 gets from Cantera's ideal-gas
 // phase: NASA7 polynomials (T <= T_mid uses the low range), e = sum Y_k e_k(T),
 // p = rho R T / W, frozen sound speed a = sqrt(cp/cv R T / W).  The UV inversion
-// is a Newton solve on T.  It first iterates in FP32 (cheap on this part) from
-// the caller's guess, then finishes in FP64 until the correction is below
-// 1e-10 T, which leaves T converged to rounding: the FP64 answer does not depend
-// on the guess or on the FP32 phase.
+// is a Newton solve on T.  It first iterates in FP32 (cheap on this part), then
+// finishes in FP64, which leaves T converged to rounding: the FP64 answer does not
+// depend on the guess or on the FP32 phase.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include "hf_fp64.cuh"
 #include "mech_h2li.h"
 
 namespace hf {
@@ -63,32 +63,58 @@ constexpr Nasa make_nasa() {
 __device__ constexpr Nasa D_NASA = make_nasa();
 constexpr double TMID = 1000.0;  // T_MID is 1000 K for every species of the table
 
+// Coefficients per unit mass density (c_kj / W_k), for weights q_k = rho Y_k.
+constexpr ECoef make_ecoef_mass() {
+    ECoef e = make_ecoef();
+    for (int r = 0; r < 2; ++r)
+        for (int k = 0; k < NS_MAX; ++k)
+            for (int j = 0; j < 6; ++j) e.c[r][k][j] /= MW[k];
+    return e;
+}
+__device__ constexpr ECoef D_ECOEF_MASS = make_ecoef_mass();
+// e_k(T) W_k / R at the temperatures that bracket the solve, per mole and per mass
+constexpr double T_LO = 250.0, T_HI = 5000.0;
+struct EAt { double lo[NS_MAX], mid[NS_MAX], hi[NS_MAX]; };
+constexpr double ecoef_at(const double (&c)[6], double T) {
+    return ((((c[4] * T + c[3]) * T + c[2]) * T + c[1]) * T + c[0]) * T + c[5];
+}
+constexpr EAt make_eat(const ECoef& e) {
+    EAt a{};
+    for (int k = 0; k < NS_MAX; ++k) {
+        a.lo[k] = ecoef_at(e.c[0][k], T_LO);
+        a.mid[k] = ecoef_at(e.c[0][k], TMID);
+        a.hi[k] = ecoef_at(e.c[1][k], T_HI);
+    }
+    return a;
+}
+__device__ constexpr EAt D_EAT = make_eat(make_ecoef());
+__device__ constexpr EAt D_EAT_MASS = make_eat(make_ecoef_mass());
+
 // Mixture polynomial of one NASA range: e(T)/R = sum_j m[j] T^(j+1) + m[5], with
-// m[j] = sum_k z_k c_kj and z_k = Y_k / W_k.
-template <int NS, int RG>
-__device__ __forceinline__ void mix_coef_r(const double* z, double* m) {
+// m[j] = sum_k w_k c_kj for weights w_k: moles (z_k = Y_k / W_k, or concentrations) or,
+// with MASS, partial densities.  Coefficients that are zero in the table (the atoms H and
+// AR have constant heat capacity) take no instruction.
+template <int NS, int RG, bool MASS = false>
+__device__ __forceinline__ void mix_coef_r(const double* w, double* m) {
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
         double s = 0.0;
+        bool first = true;
 #pragma unroll
-        for (int k = 0; k < NS; ++k) s = fma(z[k], D_ECOEF.c[RG][k][j], s);
+        for (int k = 0; k < NS; ++k) {
+            const double c = MASS ? D_ECOEF_MASS.c[RG][k][j] : D_ECOEF.c[RG][k][j];
+            if (c != 0.0) {
+                s = first ? w[k] * c : fma(w[k], c, s);
+                first = false;
+            }
+        }
         m[j] = s;
     }
 }
-template <int NS>
-__device__ __forceinline__ void mix_coef(const double* z, int range, double* m) {
-    if (range == 0) mix_coef_r<NS, 0>(z, m);
-    else mix_coef_r<NS, 1>(z, m);
-}
-template <int NS, int RG>
-__device__ __forceinline__ void mix_coef_f(const double* z, float* m) {
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-        float s = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) s = fmaf((float)z[k], (float)D_ECOEF.c[RG][k][j], s);
-        m[j] = s;
-    }
+template <int NS, bool MASS = false>
+__device__ __forceinline__ void mix_coef(const double* w, int range, double* m) {
+    if (range == 0) mix_coef_r<NS, 0, MASS>(w, m);
+    else mix_coef_r<NS, 1, MASS>(w, m);
 }
 // e/R and cv/R from mixture coefficients
 __device__ __forceinline__ double poly_e(const double* m, double T) {
@@ -104,16 +130,157 @@ __device__ __forceinline__ float poly_cv_f(const float* m, float T) {
     return fmaf(T, fmaf(T, fmaf(T, fmaf(T, 5.0f * m[4], 4.0f * m[3]), 3.0f * m[2]), 2.0f * m[1]), m[0]);
 }
 
-// Solves e(T) = e_target for the composition z (z_k = Y_k/W_k).  T holds the
-// starting guess on entry and the converged temperature on exit.  m receives the
-// FP64 mixture coefficients of the range that T ends in (for cv afterwards).
+// The UV inversion for any state: FP64 Newton from T until the applied correction is below
+// 1e-10 T (quadratic convergence leaves T at rounding level).  Inside the small jump of
+// e(T) at T_mid (no root), two consecutive sub-kelvin flips across T_mid return T_mid.
 // Returns false when the iteration does not converge to a finite positive T.
-// The FP32 phase pays even from a warm guess (the previous right-hand side's T): it
-// leaves one FP64 iteration to do instead of two or three.
-template <int NS>
-__device__ __forceinline__ bool solve_T(const double* z, double e_target, double& T, double* m) {
+template <int NS, bool MASS>
+__device__ __forceinline__ bool solve_T_any(const double* w, double et, double& T, double* m) {
     if (!(T > 0.0) || !(T < 1e5)) T = 1000.0;
-    // FP32 phase: both ranges, Newton until |dT| <= 1e-5 T.
+    int range = T <= TMID ? 0 : 1;
+    mix_coef<NS, MASS>(w, range, m);
+    int flips = 0;
+    for (int it = 0; it < 100; ++it) {
+        const int r = T <= TMID ? 0 : 1;
+        if (r != range) {
+            range = r;
+            mix_coef<NS, MASS>(w, range, m);
+        }
+        double dT = (et - poly_e(m, T)) / poly_cv(m, T);
+        if (!isfinite(dT)) return false;
+        dT = fmin(1000.0, fmax(-1000.0, dT));
+        double Tn = T + dT;
+        if (!(Tn > 0.0)) Tn = 0.5 * T;
+        const double step = fabs(Tn - T);
+        if (step <= 1e-10 * Tn) {
+            T = Tn;
+            const int rf = T <= TMID ? 0 : 1;
+            if (rf != range) mix_coef<NS, MASS>(w, rf, m);
+            return true;
+        }
+        flips = ((T <= TMID) != (Tn <= TMID) && step < 0.5) ? flips + 1 : 0;
+        if (flips >= 2) {
+            T = TMID;
+            mix_coef<NS, MASS>(w, 0, m);
+            return true;
+        }
+        T = Tn;
+    }
+    return false;
+}
+
+template <int NS, bool MASS>
+__device__ __noinline__ bool solve_T_slow(const double* w, double et, double& T, double* m, double& cv) {
+    if (!solve_T_any<NS, MASS>(w, et, T, m)) return false;
+    cv = poly_cv(m, T);
+    return true;
+}
+
+// Solves e(T) = R et for the weights w (moles, or with MASS partial densities).  T holds
+// the starting guess on entry (any value) and the converged temperature on exit; m the
+// FP64 mixture coefficients of its range, cv the heat capacity poly_cv(m, T).
+//
+// FP64 instructions are what this costs, so one FP64 Newton step of second order replaces
+// the iteration to 1e-10: e(T0) against its values at T_LO, T_MID and T_HI in FP32 picks
+// the range and a secant guess, FP32 Newton steps converge to FP32 accuracy (T within
+// about 1e-6), and with r = et - e(T0) the FP64 step
+//     T = T0 + d - (cv'/2cv) d^2,  d = r / cv
+// leaves an error of order (d/T)^3, below rounding for d <= 4e-6 T.  The mixture
+// coefficients (a sum over species for each power of T) are most of what is left: 90 FP64
+// instructions a solve.  States near T_mid, outside [T_LO, T_HI], or whose FP32 phase does
+// not settle take solve_T_any.
+template <int NS, bool MASS = false>
+__device__ __forceinline__ bool solve_T(const double* w, double et, double& T, double* m, double& cv) {
+    float t, etf = fp_to_f32(et);
+    bool low;
+    {
+        float lo = 0.0f, mid = 0.0f, hi = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            const float f = fp_to_f32(w[k]);
+            lo = fmaf(f, (float)(MASS ? D_EAT_MASS.lo[k] : D_EAT.lo[k]), lo);
+            mid = fmaf(f, (float)(MASS ? D_EAT_MASS.mid[k] : D_EAT.mid[k]), mid);
+            hi = fmaf(f, (float)(MASS ? D_EAT_MASS.hi[k] : D_EAT.hi[k]), hi);
+        }
+        low = etf <= mid;
+        t = low ? (float)T_LO + (etf - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
+                : (float)TMID + (etf - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
+        const float g = fp_to_f32(T);  // a guess on the same side of T_mid replaces the secant's
+        if (g > 200.0f && g < 6000.0f && (g <= (float)TMID) == low && g != (float)TMID) t = g;
+    }
+    if (low) mix_coef_r<NS, 0, MASS>(w, m);
+    else mix_coef_r<NS, 1, MASS>(w, m);
+    float mf[6], dt = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) mf[j] = fp_to_f32(m[j]);
+    bool fine = false;
+    for (int it = 0; it < 12; ++it) {
+        dt = (etf - poly_e_f(mf, t)) * fp_rcp_seed(poly_cv_f(mf, t));
+        t += dt;
+        fine = fabsf(dt) <= 1e-5f * t;
+        if (fine || !(fabsf(dt) < 1e4f)) break;
+    }
+    const float edge = 0.02f;
+    fine = fine && (low ? t > (float)T_LO && t < (float)TMID - edge : t > (float)TMID + edge && t < (float)T_HI);
+    if (fine) {
+        const double T0 = fp_from_f32(t);
+        double p = m[4];  // Horner: e, and by synthetic division its first two derivatives
+        double d1 = p;
+        p = fma(p, T0, m[3]);
+        double d2 = d1;
+        d1 = fma(d1, T0, p);
+        p = fma(p, T0, m[2]);
+        d2 = fma(d2, T0, d1);
+        d1 = fma(d1, T0, p);
+        p = fma(p, T0, m[1]);
+        d2 = fma(d2, T0, d1);
+        d1 = fma(d1, T0, p);
+        p = fma(p, T0, m[0]);
+        d2 = fma(d2, T0, d1);
+        d1 = fma(d1, T0, p);
+        p = fma(p, T0, m[5]);
+        const double r = et - p;
+        const double r0 = fp_from_f32(fp_rcp_seed(fp_to_f32(d1)));
+        const double d = r * fma(r0, fma(-d1, r0, 1.0), r0);
+        const float df = fp_to_f32(d), h = fp_to_f32(d2) * fp_to_f32(r0);  // d2 = cv'/2
+        if (fabsf(df) <= 4e-6f * t) {
+            const double dT = fma(d, fp_from_f32(-h * df), d);
+            T = T0 + dT;
+            // cv(T0 + dT) = cv + cv' dT + cv''/2 dT^2, the last term in FP32
+            const float d3 = fmaf(t, fmaf(t, 10.0f * mf[4], 4.0f * mf[3]), mf[2]);  // cv''/6
+            cv = fma(dT, fma(2.0, d2, fp_from_f32(3.0f * d3 * df)), d1);
+            return true;
+        }
+    }
+    // through copies, so that the arrays of the fast path stay in registers
+    double ws[NS], ms[6], Ts = fine ? fp_from_f32(t) : T, cvs = 0.0;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) ws[k] = w[k];
+    const bool ok = solve_T_slow<NS, MASS>(ws, et, Ts, ms, cvs);
+#pragma unroll
+    for (int j = 0; j < 6; ++j) m[j] = ms[j];
+    T = Ts;
+    cv = cvs;
+    return ok;
+}
+
+// The same for a specific energy e (J/kg) and weights z_k = Y_k / W_k, from a warm guess:
+// FP32 Newton with both ranges' coefficients, then solve_T_any (two FP64 iterations).  Less
+// code than the form above, which is what the chemistry kernel, bound by instruction
+// fetch, needs.
+template <int NS, int RG>
+__device__ __forceinline__ void mix_coef_f(const double* z, float* m) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        float s = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) s = fmaf((float)z[k], (float)D_ECOEF.c[RG][k][j], s);
+        m[j] = s;
+    }
+}
+template <int NS>
+__device__ __forceinline__ bool solve_T_iter(const double* z, double e_target, double& T, double* m) {
+    if (!(T > 0.0) || !(T < 1e5)) T = 1000.0;
     {
         float mlo[6], mhi[6];
         mix_coef_f<NS, 0>(z, mlo);
@@ -131,124 +298,153 @@ __device__ __forceinline__ bool solve_T(const double* z, double e_target, double
         }
         if (t > 0.0f && t < 1e5f) T = (double)t;
     }
-    // FP64 phase: stop once the applied correction is below 1e-10 T (quadratic
-    // convergence leaves T at rounding level).  Inside the small jump of e(T) at
-    // T_mid (no root), two consecutive sub-kelvin flips across T_mid return T_mid.
-    const double et = e_target * (1.0 / RU);
-    int range = T <= TMID ? 0 : 1;
-    mix_coef<NS>(z, range, m);
-    int flips = 0;
-    for (int it = 0; it < 60; ++it) {
-        const int r = T <= TMID ? 0 : 1;
-        if (r != range) {
-            range = r;
-            mix_coef<NS>(z, range, m);
-        }
-        double dT = (et - poly_e(m, T)) / poly_cv(m, T);
-        if (!isfinite(dT)) return false;
-        dT = fmin(1000.0, fmax(-1000.0, dT));
-        double Tn = T + dT;
-        if (!(Tn > 0.0)) Tn = 0.5 * T;
-        const double step = fabs(Tn - T);
-        if (step <= 1e-10 * Tn) {
-            T = Tn;
-            const int rf = T <= TMID ? 0 : 1;
-            if (rf != range) mix_coef<NS>(z, rf, m);
-            return true;
-        }
-        flips = ((T <= TMID) != (Tn <= TMID) && step < 0.5) ? flips + 1 : 0;
-        if (flips >= 2) {
-            T = TMID;
-            mix_coef<NS>(z, 0, m);
-            return true;
-        }
-        T = Tn;
-    }
-    return false;
+    return solve_T_any<NS, false>(z, e_target * (1.0 / RU), T, m);
 }
 
 struct Props { double p, a, T; };
 
+// The terms of the EOS that the face fluxes use as well.
+struct Prim { double rho, ir; };
+
+// The conditions of an admissible state that need no temperature: finite, rho > 0, no
+// negative partial density.  On bit patterns: with no negative q_k, rho = sum q_k is a
+// NaN or infinite if and only if some q_k is.
+template <int NS>
+__device__ __forceinline__ bool state_ok(const double* q, double rho) {
+    bool neg = false;
+    unsigned top = fp_abs_hi(rho);
+#pragma unroll
+    for (int k = 0; k < NS; ++k) neg = neg || fp_neg(q[k]);
+#pragma unroll
+    for (int n = NS; n < NS + 3; ++n) top = max(top, fp_abs_hi(q[n]));
+    return !neg && top < 0x7ff00000u && !fp_zero(rho) && __double2hiint(rho) >= 0;
+}
+
 // physics.cpp:4-15 for a state held in registers.  Returns false when the state
 // is inadmissible (non-finite, rho <= 0, a negative partial density, or an EOS
-// solve that fails).  T_guess seeds the UV inversion.
+// solve that fails).  T_guess seeds the UV inversion.  In units of volume: with
+// M_j = sum_k q_k c_kj / W_k the energy equation is sum_j M_j T^(j+1) + M_5 =
+// (E - |m|^2 / 2 rho) / R, so no mass fractions are formed.
+template <int NS>
+__device__ __forceinline__ bool properties(const double* q, Props& s, double T_guess, Prim& pr) {
+    double rho = q[0];
+#pragma unroll
+    for (int k = 1; k < NS; ++k) rho += q[k];
+    if (!state_ok<NS>(q, rho)) return false;
+    const double ir = fp_rcp(rho);
+    double zs = 0.0;  // sum_k q_k / W_k
+#pragma unroll
+    for (int k = 0; k < NS; ++k) zs = k ? fma(q[k], INVW.v[k], zs) : q[k] * INVW.v[k];
+    const double ke = fma(q[NS], q[NS], q[NS + 1] * q[NS + 1]) * ir;
+    const double et = fma(-0.5, ke, q[NS + 2]) * (1.0 / RU);
+    double T = T_guess, m[6], cv;
+    if (!solve_T<NS, true>(q, et, T, m, cv)) return false;
+    pr.rho = rho;
+    pr.ir = ir;
+    s.T = T;
+    s.p = RU * T * zs;
+    // a^2 = (cv + zs) / cv * p / rho = A / cv; a = A / sqrt(A cv)
+    const double A = (cv + zs) * (s.p * ir), D = A * cv;
+    if (__double2hiint(D) > 0 && fp_seedable(D)) {
+        const double y = fp_from_f32(fp_rsqrt_seed(fp_to_f32(D)));
+        const double h = A * y, e = fma(-(D * y), y, 1.0);
+        const float f = fp_to_f32(e);
+        s.a = fma(h, fma(0.5, e, fp_from_f32(0.375f * f * f)), h);
+    } else {
+        s.a = sqrt(A / cv);
+    }
+    return fp_pos(s.T) && fp_pos(s.p) && fp_pos(s.a) && fp_finite(s.a);
+}
 template <int NS>
 __device__ __forceinline__ bool properties(const double* q, Props& s, double T_guess) {
-    bool ok = true;
-    double rho = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        rho += q[k];
-        ok = ok && (q[k] >= 0.0);
-    }
-#pragma unroll
-    for (int n = NS; n < NS + 3; ++n) ok = ok && isfinite(q[n]);
-    ok = ok && isfinite(rho) && (rho > 0.0);
-    if (!ok) return false;
-    const double ir = 1.0 / rho;
-    double z[NS];
-    double zs = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        z[k] = q[k] * ir * INVW.v[k];
-        zs += z[k];
-    }
-    const double u = q[NS] * ir, v = q[NS + 1] * ir;
-    const double e = q[NS + 2] * ir - 0.5 * (u * u + v * v);
-    double T = T_guess, m[6];
-    if (!solve_T<NS>(z, e, T, m)) return false;
-    const double cvR = poly_cv(m, T);  // cv/R per unit mass (times W units)
-    const double cpR = cvR + zs;
-    s.T = T;
-    s.p = rho * RU * T * zs;
-    s.a = sqrt(cpR / cvR * RU * T * zs);
-    return s.T > 0.0 && s.p > 0.0 && s.a > 0.0 && isfinite(s.a);
+    Prim pr;
+    return properties<NS>(q, s, T_guess, pr);
 }
 
-// physics.cpp:40-44, one component
+// properties<NS>(q, ...) as a yes or no, without FP64 instructions where the answer is
+// clear.  The energy equation e(T) = et has cv > 0 on [T_LO, T_HI] for every species (and
+// cv within a factor of two of its value at T_mid on either side, so that Newton's steps
+// contract): when et lies between the energies at T_LO and T_HI by more than FP32's
+// rounding, there is a root between them, the solve finds it and p and a are positive.
+// Anything else is left to properties().
+template <int NS>
+__device__ __forceinline__ bool admissible_state(const double* q, double T_guess) {
+    bool neg = false, mass = false;
+    unsigned top = 0;
+    float lo = 0.0f, hi = 0.0f, mag = 0.0f, rho = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        neg = neg || fp_neg(q[k]);
+        top = max(top, fp_abs_hi(q[k]));
+        const float f = fp_to_f32(q[k]);
+        rho += f;
+        lo = fmaf(f, (float)D_EAT_MASS.lo[k], lo);
+        hi = fmaf(f, (float)D_EAT_MASS.hi[k], hi);
+        mag = fmaf(f, fmaxf(fabsf((float)D_EAT_MASS.lo[k]), fabsf((float)D_EAT_MASS.hi[k])), mag);
+    }
+#pragma unroll
+    for (int n = NS; n < NS + 3; ++n) top = max(top, fp_abs_hi(q[n]));
+    mass = rho > 1e-12f && rho < 1e12f;
+    if (!neg && mass && top < 0x7ff00000u) {
+        const float mu = fp_to_f32(q[NS]), mv = fp_to_f32(q[NS + 1]), E = fp_to_f32(q[NS + 2]);
+        const float ke = 0.5f * fmaf(mu, mu, mv * mv) * fp_rcp_seed(rho);
+        const float et = (E - ke) * (float)(1.0 / RU);
+        const float err = 1e-5f * (mag + (fabsf(E) + ke) * (float)(1.0 / RU));
+        if (et - err > lo && et + err < hi) return true;
+    }
+    Props p;
+    return properties<NS>(q, p, T_guess);
+}
+
+// physics.cpp:40-44, one component: x y > 0 ? copysign(min(|x|, |y|), x) : 0, from the bit
+// patterns.  The product of two numbers of one sign is positive unless it underflows or
+// one is a NaN; those cases are decided by the product itself.
 __device__ __forceinline__ double minmod(double x, double y) {
-    return x * y > 0.0 ? copysign(fmin(fabs(x), fabs(y)), x) : 0.0;
+    const unsigned hx = fp_abs_hi(x), hy = fp_abs_hi(y);
+    const unsigned long long ax = fp_abs_bits(x), ay = fp_abs_bits(y);
+    const unsigned long long lo = ax < ay ? ax : ay;
+    bool pos = (__double2hiint(x) ^ __double2hiint(y)) >= 0;
+    if (hx + hy < 0x3cf00000u ? lo != 0 : max(hx, hy) >= 0x7ff00000u) pos = fp_prod_pos_lib(x, y);
+    pos = pos && lo != 0;
+    return __hiloint2double(pos ? (int)((unsigned)(lo >> 32) | ((unsigned)__double2hiint(x) & 0x80000000u)) : 0,
+                            pos ? (int)(unsigned)lo : 0);
 }
 
-// physics.cpp:17-38: multispecies HLLC with Davis speeds in direction n (NS or NS+1).
+// physics.cpp:17-38: multispecies HLLC with Davis speeds in direction n (NS or NS+1).  In
+// the star region every advected component's flux is q (v + s (scale - 1)).  dl, dr:
+// density and its reciprocal on each side.
 template <int NS, int N>
 __device__ __forceinline__ void hllc(const double* l, const double* r, const Props& pl, const Props& pr,
-                                     double* f) {
+                                     const Prim& dl_, const Prim& dr_, double* f) {
     constexpr int E = NS + 2;
-    double rl = 0.0, rr = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) { rl += l[k]; rr += r[k]; }
-    const double ul = l[N] / rl, ur = r[N] / rr;
-    const double sl = fmin(ul - pl.a, ur - pr.a), sr = fmax(ul + pl.a, ur + pr.a);
-    if (sl >= 0.0 || sr <= 0.0) {
-        const bool useL = sl >= 0.0;
-        const double* q = useL ? l : r;
-        const double v = useL ? ul : ur, p = useL ? pl.p : pr.p;
-#pragma unroll
-        for (int m = 0; m < NS + 3; ++m) f[m] = v * q[m];
-        f[N] += p;
-        f[E] += p * v;
-        return;
+    const double rl = dl_.rho, rr = dr_.rho;
+    const double ul = l[N] * dl_.ir, ur = r[N] * dr_.ir;
+    const double sl = fp_min(ul - pl.a, ur - pr.a), sr = fp_max(ul + pl.a, ur + pr.a);
+    const bool allL = fp_ge0(sl), allR = !allL && !fp_pos(sr);
+    const double wl = sl - ul, wr = sr - ur;
+    const double dl = rl * wl, dr = rr * wr;
+    double sm = 0.0;
+    bool left = allL;
+    if (!allL && !allR) {
+        sm = fp_div((pr.p - pl.p) + fma(dl, ul, -dr * ur), dl - dr);
+        left = fp_ge0(sm);
     }
-    const double dl = rl * (sl - ul), dr = rr * (sr - ur);
-    const double sm = (pr.p - pl.p + dl * ul - dr * ur) / (dl - dr);
-    const bool left = sm >= 0.0;
-    const double* q = left ? l : r;
-    const double v = left ? ul : ur, s = left ? sl : sr, p = left ? pl.p : pr.p, rq = left ? rl : rr;
-    const double scale = (s - v) / (s - sm);
-    double rs = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) rs += q[k] * scale;
-    const double estar = q[E] * scale + rs * (sm - v) * (sm + p / (rq * (s - v)));
+    const double v = left ? ul : ur, p = left ? pl.p : pr.p;
+    double qn = left ? l[N] : r[N], qe = left ? l[E] : r[E];
+    double wgt = v, fn = fma(v, qn, p), fe = v * (qe + p);
+    if (!allL && !allR) {
+        const double s = left ? sl : sr, w = left ? wl : wr, d = left ? dl : dr, rq = left ? rl : rr;
+        const double scale = fp_div(w, s - sm);
+        const double rs = rq * scale;
+        const double estar = fma(qe, scale, rs * (sm - v) * (sm + fp_div(p, d)));
+        wgt = fma(s, scale - 1.0, v);
+        fn = fma(s, fma(rs, sm, -qn), fn);
+        fe = fma(s, estar - qe, fe);
+    }
 #pragma unroll
     for (int m = 0; m < NS + 3; ++m) {
-        double st = q[m] * scale;
-        if (m == N) st = rs * sm;
-        if (m == E) st = estar;
-        double fl = v * q[m];
-        if (m == N) fl += p;
-        if (m == E) fl += p * v;
-        f[m] = fl + s * (st - q[m]);
+        const double q = left ? l[m] : r[m];
+        f[m] = m == N ? fn : m == E ? fe : q * wgt;
     }
 }
 

@@ -94,11 +94,9 @@ hf_status stage_fwd(hf_flow_tape* t, double* in, const double* old, double* out,
                     bool replay, cudaStream_t s) {
     hf_status r = hf_fill_ghosts(t->ctx, &t->L, &t->P, 1, in, s);
     if (r != HF_OK) return r;
-    int64_t bad = -1;
-    if (replay) return hf_flux_update(t->ctx, &t->L, &t->P, 1, in, old, out, nullptr, nullptr, h, fo, HF_FLUX_PLAIN,
-                                      &bad, s);
+    if (replay) return hf::record_flux_update(t->ctx, &t->L, &t->P, in, old, out, h, fo, s);
     for (int f = 0; f < 2; ++f) {
-        r = hf_flux_update(t->ctx, &t->L, &t->P, 1, in, old, out, nullptr, nullptr, h, f, HF_FLUX_PLAIN, &bad, s);
+        r = hf::record_flux_update(t->ctx, &t->L, &t->P, in, old, out, h, f, s);
         if (r == HF_OK) {
             fo = (unsigned char)f;
             return HF_OK;
@@ -204,7 +202,7 @@ hf_status hf_flow_record(hf_ctx* ctx, const hf_level* level, const double* U0, i
     hf_status r = (cur && nxt && w[0] && w[1] && w[2] && w[3]) ? copy_interior(t, cur, U0, s, true) : HF_ERR_CUDA;
     for (int n = 0; r == HF_OK && n < nsteps; ++n) {
         if (n % t->K == 0) r = cuda_status(cudaMemcpyAsync(t->ck[n / t->K], cur, t->bytes, cudaMemcpyDeviceToDevice, s));
-        if (r == HF_OK && !dts) r = hf_cfl_dt(ctx, &t->L, &t->P, 1, cur, cfl, &t->dts[n], s);
+        if (r == HF_OK && !dts) r = hf::record_cfl_dt(ctx, &t->L, &t->P, cur, cfl, &t->dts[n], s);
         if (r == HF_OK) r = step_fwd(t, n, cur, w, nxt, false, s);
         std::swap(cur, nxt);
     }

@@ -14,7 +14,7 @@
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cstring>
-#include "hf_device.cuh"
+#include "hf_record.cuh"
 #include "hf_internal.h"
 
 namespace hf {
@@ -170,7 +170,13 @@ cudaError_t launch_fill(int ns, const Level& L, const hf_patch* ph, const hf_pat
 
 // ---------------------------------------------------------------- face flux (shared)
 // One face: 4-cell stencil values are fetched by get(k, n), k = 0..3 for qa..qd.
-template <int NS, int D, class Get>
+// REC: the arithmetic of recorded runs (hf_record.cuh).
+template <int NS, bool REC>
+__device__ __forceinline__ bool face_props(const double* q, Props& p, Prim& d) {
+    if constexpr (REC) return rec::properties<NS>(q, p, 1000.0);
+    else return properties<NS>(q, p, 0.0, d);
+}
+template <int NS, int D, bool REC, class Get>
 __device__ __forceinline__ bool face_flux(const Level& L, int gi, int gj, int first_order, Get get, double* f) {
     constexpr int NV = NS + 3;
     double lq[NV], rq[NV];
@@ -181,22 +187,25 @@ __device__ __forceinline__ bool face_flux(const Level& L, int gi, int gj, int fi
             lq[n] = qb;
             rq[n] = qc;
         } else {
-            lq[n] = qb + 0.5 * minmod(qb - qa, qc - qb);
-            rq[n] = qc - 0.5 * minmod(qc - qb, qd - qc);
+            const double mid = qc - qb;
+            lq[n] = fma(0.5, minmod(qb - qa, mid), qb);
+            rq[n] = fma(-0.5, minmod(mid, qd - qc), qc);
         }
     }
     Props pl, pr;
-    if (!properties<NS>(lq, pl, 1000.0)) {
+    Prim dl, dr;
+    if (!face_props<NS, REC>(lq, pl, dl)) {
 #pragma unroll
         for (int n = 0; n < NV; ++n) lq[n] = get(1, n);
-        if (!properties<NS>(lq, pl, 1000.0)) return false;
+        if (!face_props<NS, REC>(lq, pl, dl)) return false;
     }
-    if (!properties<NS>(rq, pr, 1000.0)) {
+    if (!face_props<NS, REC>(rq, pr, dr)) {
 #pragma unroll
         for (int n = 0; n < NV; ++n) rq[n] = get(2, n);
-        if (!properties<NS>(rq, pr, 1000.0)) return false;
+        if (!face_props<NS, REC>(rq, pr, dr)) return false;
     }
-    hllc<NS, NS + D>(lq, rq, pl, pr, f);
+    if constexpr (REC) rec::hllc<NS, NS + D>(lq, rq, pl, pr, f);
+    else hllc<NS, NS + D>(lq, rq, pl, pr, dl, dr, f);
     // wall-flux override, BlockAMR.cpp:224-229
     const bool loWall = !L.periodic[D] && (L.lo[D] == HF_BC_REFLECTING || L.lo[D] == HF_BC_WEDGE);
     const bool hiWall = !L.periodic[D] && L.hi[D] == HF_BC_REFLECTING;
@@ -214,8 +223,20 @@ __device__ __forceinline__ bool face_flux(const Level& L, int gi, int gj, int fi
 }
 
 // ---------------------------------------------------------------- plain form
+// All kernels of this path are bound by the FP64 pipe (80% active; 64 cycles of an SM
+// sub-partition per warp instruction, hf_fp64.cuh), so what they cost is their FP64
+// instruction count, measured on 1024 x 256 cells (10 species):
+//   face kernels   361 a face (1105 when limiter, comparisons and conversions were FP64
+//                  instructions and an EOS solve took two FP64 Newton steps): 0.206 ms a
+//                  direction against 0.595; of them about 230 are the two EOS solves, 65 the
+//                  reconstruction
+//   update         52 a cell (438 with an EOS solve to validate): 0.033 against 0.230 ms
+//   CFL            118 a cell (434): 0.070 against 0.229 ms
+// The face kernels are held to 128 registers (4 blocks an SM; 16 bytes spilled): 13.5 warps
+// in flight instead of 10.5 at 156 registers hide the integer work, 3.56 against 3.66 ms for
+// a flow of 2048 x 512 cells.
 // Face idx of direction D of patch P into F (component stride = the patch's face count).
-template <int NS, int D>
+template <int NS, int D, bool REC = false>
 __device__ __forceinline__ void face_one(const Level& L, const hf_patch& P, const double* __restrict__ U,
                                          double* __restrict__ F, int first_order, int64_t cell_base, DevStatus* st,
                                          int64_t idx) {
@@ -227,7 +248,7 @@ __device__ __forceinline__ void face_one(const Level& L, const hf_patch& P, cons
         return D == 0 ? v.get(fi - 2 + k, fj, n) : v.get(fi, fj - 2 + k, n);
     };
     double f[NS + 3];
-    if (!face_flux<NS, D>(L, P.ilo + fi, P.jlo + fj, first_order, get, f)) {
+    if (!face_flux<NS, D, REC>(L, P.ilo + fi, P.jlo + fj, first_order, get, f)) {
         flag(st, ST_FACE_BAD, cell_base + (int64_t)min(fj, P.ny - 1) * P.nx + min(fi, P.nx - 1));
 #pragma unroll
         for (int n = 0; n < NS + 3; ++n) f[n] = 0.0;
@@ -238,17 +259,39 @@ __device__ __forceinline__ void face_one(const Level& L, const hf_patch& P, cons
 }
 
 template <int NS, int D>
-__global__ void __launch_bounds__(128) k_face_plain(Level L, hf_patch P, const double* __restrict__ U,
+__global__ void __launch_bounds__(128, 4) k_face_plain(Level L, hf_patch P, const double* __restrict__ U,
                                                     double* __restrict__ F, int first_order, int64_t cell_base,
                                                     DevStatus* st) {
     if (st->abort_run) return;  // an earlier step of this device-resident run failed
     face_one<NS, D>(L, P, U, F, first_order, cell_base, st, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+template <int NS, int D>
+__global__ void __launch_bounds__(128) k_face_record(Level L, hf_patch P, const double* __restrict__ U,
+                                                     double* __restrict__ F, int first_order, DevStatus* st) {
+    face_one<NS, D, true>(L, P, U, F, first_order, 0, st, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+}
+// the face kernels of a recorded run's stage
+cudaError_t launch_faces_record(int ns, const Level& L, const hf_patch& P, const double* U, double* fx, double* fy,
+                                int first_order, DevStatus* st, cudaStream_t s, int64_t* launches) {
+    const int bs = 128;
+    const unsigned gx = (unsigned)(((int64_t)(P.nx + 1) * P.ny + bs - 1) / bs);
+    const unsigned gy = (unsigned)(((int64_t)P.nx * (P.ny + 1) + bs - 1) / bs);
+    if (ns == 9) {
+        k_face_record<9, 0><<<gx, bs, 0, s>>>(L, P, U, fx, first_order, st);
+        k_face_record<9, 1><<<gy, bs, 0, s>>>(L, P, U, fy, first_order, st);
+    } else {
+        k_face_record<10, 0><<<gx, bs, 0, s>>>(L, P, U, fx, first_order, st);
+        k_face_record<10, 1><<<gy, bs, 0, s>>>(L, P, U, fy, first_order, st);
+    }
+    *launches += 2;
+    return cudaGetLastError();
+}
+
 // All patches of a level in one launch: patch blockIdx.y, its x/y face arrays at
 // off[3p], off[3p+1] of FX/FY and its first cell's index at off[3p+2].
 template <int NS, int D>
-__global__ void __launch_bounds__(128) k_face_multi(Level L, const hf_patch* __restrict__ patches,
+__global__ void __launch_bounds__(128, 4) k_face_multi(Level L, const hf_patch* __restrict__ patches,
                                                     const int64_t* __restrict__ off, const double* __restrict__ U,
                                                     double* __restrict__ F, int first_order, DevStatus* st) {
     if (st->abort_run) return;
@@ -268,17 +311,16 @@ __device__ __forceinline__ void finish_cell(double* q, const double* __restrict_
     constexpr int NV = NS + 3;
     bool neg = false;
 #pragma unroll
-    for (int k = 0; k < NS; ++k) neg = neg || (q[k] < 0.0);
-    Props p;
+    for (int k = 0; k < NS; ++k) neg = neg || fp_neg(q[k]);
     if (neg) {
         flag(st, ST_NEGATIVE, cell);
-    } else if (!properties<NS>(q, p, 1000.0)) {
+    } else if (!admissible_state<NS>(q, 0.0)) {
         flag(st, ST_STAGE_BAD, cell);
     }
     if (Uold) {
 #pragma unroll
-        for (int n = 0; n < NV; ++n) q[n] = 0.5 * Uold[gidx + n * cstride] + 0.5 * q[n];
-        if (!neg && !properties<NS>(q, p, 1000.0)) flag(st, ST_COMBINE_BAD, cell);
+        for (int n = 0; n < NV; ++n) q[n] = fp_half(Uold[gidx + n * cstride] + q[n]);
+        if (!neg && !admissible_state<NS>(q, 0.0)) flag(st, ST_COMBINE_BAD, cell);
     }
 #pragma unroll
     for (int n = 0; n < NV; ++n) Uout[gidx + n * cstride] = q[n];
@@ -343,11 +385,17 @@ template <int NS>
 static cudaError_t flux_plain_impl(const Level& L, const hf_patch& P, const double* Uin, const double* Uold,
                                    double* Uout, double* fx, double* fy, double h, int first_order,
                                    int64_t cell_base, DevStatus* st, cudaStream_t s, int64_t* launches,
-                                   const double* hdev) {
+                                   const double* hdev, bool record) {
     const int bs = 128;
     const int64_t nfx = (int64_t)(P.nx + 1) * P.ny, nfy = (int64_t)P.nx * (P.ny + 1);
-    k_face_plain<NS, 0><<<(unsigned)((nfx + bs - 1) / bs), bs, 0, s>>>(L, P, Uin, fx, first_order, cell_base, st);
-    k_face_plain<NS, 1><<<(unsigned)((nfy + bs - 1) / bs), bs, 0, s>>>(L, P, Uin, fy, first_order, cell_base, st);
+    if (record) {
+        const cudaError_t e = launch_faces_record(NS, L, P, Uin, fx, fy, first_order, st, s, launches);
+        if (e != cudaSuccess) return e;
+        *launches -= 2;
+    } else {
+        k_face_plain<NS, 0><<<(unsigned)((nfx + bs - 1) / bs), bs, 0, s>>>(L, P, Uin, fx, first_order, cell_base, st);
+        k_face_plain<NS, 1><<<(unsigned)((nfy + bs - 1) / bs), bs, 0, s>>>(L, P, Uin, fy, first_order, cell_base, st);
+    }
     const int64_t nc = (int64_t)P.nx * P.ny;
     k_update_plain<NS><<<(unsigned)((nc + bs - 1) / bs), bs, 0, s>>>(P, Uin, Uold, Uout, fx, fy, h / L.dx, h / L.dy,
                                                                      hdev, L.dx, L.dy, cell_base, st);
@@ -386,10 +434,11 @@ cudaError_t launch_flux_multi(int ns, const Level& L, const hf_patch* patches_ho
 }
 cudaError_t launch_flux_plain(int ns, const Level& L, const hf_patch& P, int, const double* Uin, const double* Uold,
                               double* Uout, double* fx, double* fy, double h, int first_order, int64_t cell_base,
-                              DevStatus* st, cudaStream_t s, int64_t* launches, const double* hdev) {
-    return ns == 9 ? flux_plain_impl<9>(L, P, Uin, Uold, Uout, fx, fy, h, first_order, cell_base, st, s, launches, hdev)
+                              DevStatus* st, cudaStream_t s, int64_t* launches, const double* hdev, bool record) {
+    return ns == 9 ? flux_plain_impl<9>(L, P, Uin, Uold, Uout, fx, fy, h, first_order, cell_base, st, s, launches, hdev,
+                                        record)
                    : flux_plain_impl<10>(L, P, Uin, Uold, Uout, fx, fy, h, first_order, cell_base, st, s, launches,
-                                         hdev);
+                                         hdev, record);
 }
 
 // ---------------------------------------------------------------- fused form
@@ -551,7 +600,7 @@ __global__ void __launch_bounds__(NTHR) k_flux_fused(const __grid_constant__ CUt
             const int fi = f % (TX + 1), fj = f / (TX + 1);
             ci = ti0 + fi; cj = tj0 + fj;
             auto get = [&](int k, int n) { return T(fi + k, fj + 2, n); };
-            ok = (ci <= P.nx && cj < P.ny) ? face_flux<NS, 0>(L, P.ilo + ci, P.jlo + cj, first_order, get, fl) : true;
+            ok = (ci <= P.nx && cj < P.ny) ? face_flux<NS, 0, false>(L, P.ilo + ci, P.jlo + cj, first_order, get, fl) : true;
             if (!ok) { for (int n = 0; n < NV; ++n) fl[n] = 0.0; }
             for (int n = 0; n < NV; ++n) sfx[(n * TY + fj) * (TX + 1) + fi] = fl[n];
         } else {
@@ -559,7 +608,7 @@ __global__ void __launch_bounds__(NTHR) k_flux_fused(const __grid_constant__ CUt
             const int fi = g % TX, fj = g / TX;
             ci = ti0 + fi; cj = tj0 + fj;
             auto get = [&](int k, int n) { return T(fi + 2, fj + k, n); };
-            ok = (ci < P.nx && cj <= P.ny) ? face_flux<NS, 1>(L, P.ilo + ci, P.jlo + cj, first_order, get, fl) : true;
+            ok = (ci < P.nx && cj <= P.ny) ? face_flux<NS, 1, false>(L, P.ilo + ci, P.jlo + cj, first_order, get, fl) : true;
             if (!ok) { for (int n = 0; n < NV; ++n) fl[n] = 0.0; }
             for (int n = 0; n < NV; ++n) sfy[(n * (TY + 1) + fj) * TX + fi] = fl[n];
         }
@@ -661,11 +710,10 @@ __global__ void k_combine(hf_patch P, const double* __restrict__ Uold, double* _
     double q[NS + 3];
 #pragma unroll
     for (int n = 0; n < NS + 3; ++n) {
-        q[n] = 0.5 * Uold[g + n * P.comp_stride] + 0.5 * U[g + n * P.comp_stride];
+        q[n] = fp_half(Uold[g + n * P.comp_stride] + U[g + n * P.comp_stride]);
         U[g + n * P.comp_stride] = q[n];
     }
-    Props p;
-    if (!properties<NS>(q, p, 1000.0)) flag(st, ST_COMBINE_BAD, cell_base + idx);
+    if (!admissible_state<NS>(q, 0.0)) flag(st, ST_COMBINE_BAD, cell_base + idx);
 }
 template <int NS>
 __device__ __forceinline__ void validate_one(const hf_patch& P, const double* __restrict__ U, int64_t cell_base,
@@ -676,8 +724,7 @@ __device__ __forceinline__ void validate_one(const hf_patch& P, const double* __
     double q[NS + 3];
 #pragma unroll
     for (int n = 0; n < NS + 3; ++n) q[n] = U[g + n * P.comp_stride];
-    Props p;
-    if (!properties<NS>(q, p, 1000.0)) flag(st, ST_STAGE_BAD, cell_base + idx);
+    if (!admissible_state<NS>(q, 0.0)) flag(st, ST_STAGE_BAD, cell_base + idx);
 }
 template <int NS>
 __global__ void k_validate(hf_patch P, const double* __restrict__ U, int64_t cell_base, DevStatus* st) {
@@ -695,7 +742,7 @@ __global__ void k_validate_multi(const hf_patch* __restrict__ patches, const int
 
 // CFL rate of cell idx of patch P (0 outside it or when inadmissible, which is flagged
 // with bad index cell_base + idx); the block's warps fold it into st->rate_bits.
-template <int NS>
+template <int NS, bool REC = false>
 __device__ __forceinline__ void cfl_one(const Level& L, const hf_patch& P, const double* __restrict__ U,
                                         int64_t cell_base, DevStatus* st, int64_t idx) {
     double rate = 0.0;
@@ -706,23 +753,26 @@ __device__ __forceinline__ void cfl_one(const Level& L, const hf_patch& P, const
 #pragma unroll
         for (int n = 0; n < NS + 3; ++n) q[n] = U[g + n * P.comp_stride];
         Props p;
-        if (!properties<NS>(q, p, 1000.0)) {
+        Prim d;
+        if (!face_props<NS, REC>(q, p, d)) {
             flag(st, ST_STAGE_BAD, cell_base + idx);
-        } else {
+        } else if constexpr (REC) {
             double rho = 0.0;
 #pragma unroll
             for (int k = 0; k < NS; ++k) rho += q[k];
             rate = (fabs(q[NS] / rho) + p.a) / L.dx + (fabs(q[NS + 1] / rho) + p.a) / L.dy;
+        } else {
+            rate = fma(fma(fabs(q[NS]), d.ir, p.a), L.rdx, fma(fabs(q[NS + 1]), d.ir, p.a) * L.rdy);
         }
     }
     // warp max then one atomic per warp (max is order independent: deterministic)
-    for (int o = 16; o > 0; o >>= 1) rate = fmax(rate, __shfl_xor_sync(0xffffffffu, rate, o));
+    for (int o = 16; o > 0; o >>= 1) rate = fp_abs_max(rate, __shfl_xor_sync(0xffffffffu, rate, o));
     if ((threadIdx.x & 31) == 0 && rate > 0.0) atomicMax(&st->rate_bits, (unsigned long long)__double_as_longlong(rate));
 }
-template <int NS>
+template <int NS, bool REC>
 __global__ void k_cfl(Level L, hf_patch P, const double* __restrict__ U, DevStatus* st) {
     if (st->abort_run) return;
-    cfl_one<NS>(L, P, U, 0, st, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    cfl_one<NS, REC>(L, P, U, 0, st, (int64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 template <int NS>
 __global__ void k_cfl_multi(Level L, const hf_patch* __restrict__ patches, const int64_t* __restrict__ base,
@@ -767,9 +817,10 @@ cudaError_t launch_cfl_multi(int ns, const Level& L, const hf_patch* ph, const h
     return cudaGetLastError();
 }
 cudaError_t launch_cfl(int ns, const Level& L, const hf_patch& P, const double* U, DevStatus* st, cudaStream_t s,
-                       int64_t* launches) {
+                       int64_t* launches, bool record) {
     const int64_t n = (int64_t)P.nx * P.ny;
-    HF_DISPATCH(ns, k_cfl)<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(L, P, U, st);
+    auto k = ns == 9 ? (record ? k_cfl<9, true> : k_cfl<9, false>) : (record ? k_cfl<10, true> : k_cfl<10, false>);
+    k<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(L, P, U, st);
     ++*launches;
     return cudaGetLastError();
 }
@@ -784,7 +835,7 @@ __global__ void k_properties(const double* __restrict__ q, int64_t stride, int64
 #pragma unroll
     for (int n = 0; n < NS + 3; ++n) s[n] = q[n * stride + i];
     Props pr{0.0, 0.0, 0.0};
-    const bool ok = properties<NS>(s, pr, 1000.0);
+    const bool ok = properties<NS>(s, pr, 0.0);
     p[i] = pr.p;
     a[i] = pr.a;
     T[i] = pr.T;
@@ -800,8 +851,13 @@ __global__ void k_hllc(const double* __restrict__ l, const double* __restrict__ 
 #pragma unroll
     for (int n = 0; n < NS + 3; ++n) { a[n] = l[n * stride + i]; b[n] = r[n * stride + i]; }
     const Props A{pl[i], pl[stride + i], pl[2 * stride + i]}, B{pr[i], pr[stride + i], pr[2 * stride + i]};
-    if (dir == 0) hllc<NS, NS>(a, b, A, B, o);
-    else hllc<NS, NS + 1>(a, b, A, B, o);
+    Prim da{a[0], 0.0}, db{b[0], 0.0};
+#pragma unroll
+    for (int n = 1; n < NS; ++n) { da.rho += a[n]; db.rho += b[n]; }
+    da.ir = fp_rcp(da.rho);
+    db.ir = fp_rcp(db.rho);
+    if (dir == 0) hllc<NS, NS>(a, b, A, B, da, db, o);
+    else hllc<NS, NS + 1>(a, b, A, B, da, db, o);
 #pragma unroll
     for (int n = 0; n < NS + 3; ++n) f[n * stride + i] = o[n];
 }
@@ -851,8 +907,7 @@ __device__ __forceinline__ void interp_one(const hf_patch& C, const double* __re
                 double child[NV];
 #pragma unroll
                 for (int n = 0; n < NV; ++n) child[n] = q[n] + theta * ((a ? 0.25 : -0.25) * sx[n] + (b ? 0.25 : -0.25) * sy[n]);
-                Props p;
-                good = properties<NS>(child, p, 1000.0);
+                good = admissible_state<NS>(child, 0.0);
             }
         if (good) { accepted = true; break; }
         theta *= 0.5;

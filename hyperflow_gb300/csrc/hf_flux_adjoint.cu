@@ -10,7 +10,7 @@
 //   gather per ghosted cell;  transpose of the ghost fill -> interior cotangents.
 // The roundoff repair of the forward (BlockAMR.cpp:299-334) is taken as the
 // identity, and validation has no derivative.
-#include "hf_device.cuh"
+#include "hf_record.cuh"
 #include "hf_internal.h"
 
 namespace hf {
@@ -34,7 +34,7 @@ struct Eos {
 template <int NS>
 __device__ __forceinline__ bool eos_fwd(const double* q, Eos<NS>& t) {
     Props pr;
-    if (!properties<NS>(q, pr, 1000.0)) return false;
+    if (!rec::properties<NS>(q, pr, 1000.0)) return false;
     double rho = 0.0;
 #pragma unroll
     for (int k = 0; k < NS; ++k) rho += q[k];

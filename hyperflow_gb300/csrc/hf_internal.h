@@ -39,6 +39,7 @@ struct Level {  // device copy of hf_level
     int nx, ny;
     int periodic[2], lo[2], hi[2];
     double dx, dy, xlo, ylo, wedge_start;
+    double rdx, rdy;  // 1/dx, 1/dy
     double inlet[13];
 };
 inline Level make_level(const hf_level& l) {
@@ -46,6 +47,7 @@ inline Level make_level(const hf_level& l) {
     d.nx = l.nx; d.ny = l.ny;
     for (int k = 0; k < 2; ++k) { d.periodic[k] = l.periodic[k]; d.lo[k] = l.bc_lo[k]; d.hi[k] = l.bc_hi[k]; }
     d.dx = l.dx; d.dy = l.dy; d.xlo = l.xlo; d.ylo = l.ylo; d.wedge_start = l.wedge_start;
+    d.rdx = 1.0 / l.dx; d.rdy = 1.0 / l.dy;
     for (int n = 0; n < 13; ++n) d.inlet[n] = l.inlet[n];
     return d;
 }
@@ -62,14 +64,22 @@ bool ctx_timing_enabled(const hf_ctx* ctx);
 void ctx_add_timing(hf_ctx* ctx, double flux_ms, double chem_ms, double other_ms, int64_t flux_launches,
                     int64_t chem_launches, int64_t other_launches);
 
+// hf_flux_update (plain form, one patch) and hf_cfl_dt in the arithmetic of recorded runs
+// (hf_record.cuh)
+hf_status record_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U_in,
+                             const double* U_old, double* U_out, double h, int first_order, void* stream);
+hf_status record_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U, double cfl,
+                        double* dt, void* stream);
+
 // Launch wrappers (hf_flux.cu)
 cudaError_t launch_fill(int ns, const Level& L, const hf_patch* patches_host, const hf_patch* patches_dev,
                         int npatch, double* U, cudaStream_t s, int64_t* launches);
-// hdev (nullable): read the stage length h from device memory instead of the argument
+// hdev (nullable): read the stage length h from device memory instead of the argument;
+// record: the arithmetic of recorded runs (hf_record.cuh)
 cudaError_t launch_flux_plain(int ns, const Level& L, const hf_patch& P, int pidx, const double* Uin,
                               const double* Uold, double* Uout, double* fx, double* fy, double h,
                               int first_order, int64_t cell_base, DevStatus* st, cudaStream_t s,
-                              int64_t* launches, const double* hdev = nullptr);
+                              int64_t* launches, const double* hdev = nullptr, bool record = false);
 // The plain form over all patches of a level in 3 launches; off_dev[3p..3p+2] = patch p's
 // x-face offset in FX, y-face offset in FY and first cell index (face arrays packed per
 // patch, component-major within a patch, as launch_flux_plain writes them).
@@ -95,7 +105,7 @@ cudaError_t launch_cfl_multi(int ns, const Level& L, const hf_patch* patches_hos
 cudaError_t launch_validate(int ns, const hf_patch& P, const double* U, int64_t cell_base, DevStatus* st,
                             cudaStream_t s, int64_t* launches);
 cudaError_t launch_cfl(int ns, const Level& L, const hf_patch& P, const double* U, DevStatus* st,
-                       cudaStream_t s, int64_t* launches);
+                       cudaStream_t s, int64_t* launches, bool record = false);
 cudaError_t launch_properties(int ns, const double* q, int64_t stride, int64_t count, double* p, double* a,
                               double* T, int32_t* status, DevStatus* st, cudaStream_t s, int64_t* launches);
 cudaError_t launch_hllc(int ns, const double* l, const double* r, const double* pl, const double* pr,

@@ -417,7 +417,7 @@ __device__ __noinline__ bool chem_rhs(double rho, double e, double& T, const dou
     double z[NS], C[NS], m[6];
     comp<NS>(y, rho, z, C);
     double Tn = T;
-    if (!solve_T<NS>(z, e, Tn, m)) return false;
+    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
     T = Tn;
     KinCtx<NS> kc;
     kin_setup<NS>(T, C, kc);
@@ -441,7 +441,7 @@ __device__ __noinline__ bool chem_jac(double rho, double e, double& T, const dou
     double z[NS], C[NS], m[6];
     comp<NS>(y, rho, z, C);
     double Tn = T;
-    if (!solve_T<NS>(z, e, Tn, m)) return false;
+    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
     T = Tn;
     KinCtx<NS> kc;
     kin_setup<NS>(T, C, kc);
@@ -477,7 +477,7 @@ __device__ __noinline__ bool chem_rhs_jac(double rho, double e, double& T, const
     double z[NS], C[NS], m[6];
     comp<NS>(y, rho, z, C);
     double Tn = T;
-    if (!solve_T<NS>(z, e, Tn, m)) return false;
+    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
     T = Tn;
     KinCtx<NS> kc;
     kin_setup<NS>(T, C, kc);
