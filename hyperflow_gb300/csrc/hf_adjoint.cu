@@ -26,7 +26,7 @@
 // of K calls is recomputed from its checkpoint, storing the state at every call
 // boundary and the tape of accepted steps (y, h, T); a segment whose tape exceeds
 // its capacity recomputes each call again from the stored boundary states.
-#include "hf_kinetics.cuh"
+#include "hf_cell.cuh"
 
 namespace hf {
 
@@ -564,8 +564,9 @@ template <int NS>
 __device__ int run_call(double* u, double dt, double rtol, double atol, double* tape, int64_t tstride, int& nrec,
                         int cap, uint32_t& clip) {
     constexpr int N = NS - 1;
-    ChemCell<NS> c;
-    int r = cell_begin<NS>(c, u, dt, rtol, atol);
+    cell::Cell<NS> c;
+    double Lu[cell::NQ * cell::NQ];
+    int r = cell::begin<NS>(c, u, dt, rtol, atol);
     while (r == CELL_CONTINUE) {
         double yp[N];
 #pragma unroll
@@ -573,7 +574,7 @@ __device__ int run_call(double* u, double dt, double rtol, double atol, double* 
         const double Tp = c.T;
         const double he = (c.t + 1.01 * c.h >= c.tend) ? c.tend - c.t : c.h;
         const int s0 = c.steps;
-        r = cell_attempt<NS>(c, rtol, atol);
+        r = cell::attempt<NS, false, 1>(c, rtol, atol, Lu);
         if (tape && c.steps > s0) {
             if (nrec < cap) {
                 double* t = tape + (int64_t)nrec * (N + 2) * tstride;
@@ -590,7 +591,7 @@ __device__ int run_call(double* u, double dt, double rtol, double atol, double* 
 #pragma unroll
     for (int k = 0; k < N; ++k)
         if (c.y[k] < 0.0) clip |= 1u << k;
-    return cell_end<NS>(c, u) ? CELL_DONE : CELL_FAIL;
+    return cell::finish<NS>(c, u) ? CELL_DONE : CELL_FAIL;
 }
 
 // dT/dy and dp/dy of the state u (y = u/rho at fixed rho, e).

@@ -19,6 +19,7 @@
 // is a register index.
 #include <atomic>
 #include <cstdlib>
+#include "hf_cell.cuh"
 #include "hf_chem_coop.cuh"
 
 namespace hf {
@@ -50,11 +51,13 @@ __global__ void __launch_bounds__(64) k_chem_plain(const double* __restrict__ U,
     if (dt_dev) dt = *dt_dev;  // interval from device memory (graph-captured steps)
     double u[NS + 3];
     load_cell<NS>(U, cs, cell_index ? cell_index[i] : i, u);
-    ChemCell<NS> c;
-    int r = cell_begin<NS>(c, u, dt_cell ? dt_cell[i] : dt, rtol, atol);
-    while (r == CELL_CONTINUE) r = cell_attempt<NS>(c, rtol, atol);
+    cell::Cell<NS> c;
+    double Lu[cell::NQ * cell::NQ];
+    c.attempts = 0;
+    int r = cell::begin<NS>(c, u, dt_cell ? dt_cell[i] : dt, rtol, atol);
+    while (r == CELL_CONTINUE) r = cell::attempt<NS, false, 1>(c, rtol, atol, Lu);
     atomicAdd(&st->steps, (unsigned long long)c.attempts);
-    if (r == CELL_DONE && cell_end<NS>(c, u)) {
+    if (r == CELL_DONE && cell::finish<NS>(c, u)) {
 #pragma unroll
         for (int n = 0; n < NS + 3; ++n) trial[n * count + i] = u[n];
         fail[i] = 0;
@@ -75,7 +78,8 @@ __global__ void __launch_bounds__(64) k_chem_persistent(const double* __restrict
                                                         double atol, double* __restrict__ trial,
                                                         int* __restrict__ fail, DevStatus* st) {
     const unsigned lane = threadIdx.x & 31;
-    ChemCell<NS> c;
+    cell::Cell<NS> c;
+    double Lu[cell::NQ * cell::NQ];
     int64_t cell = -1;
     bool active = false, drained = false;
     unsigned long long my_attempts = 0;
@@ -95,7 +99,7 @@ __global__ void __launch_bounds__(64) k_chem_persistent(const double* __restrict
                         cell = k;
                         double u[NS + 3];
                         load_cell<NS>(U, cs, cell_index ? cell_index[k] : k, u);
-                        const int r = cell_begin<NS>(c, u, dt_cell ? dt_cell[k] : dt, rtol, atol);
+                        const int r = cell::begin<NS>(c, u, dt_cell ? dt_cell[k] : dt, rtol, atol);
                         if (r == CELL_CONTINUE) active = true;
                         else report(st, fail, k, CELL_FAIL);
                     } else {
@@ -110,11 +114,11 @@ __global__ void __launch_bounds__(64) k_chem_persistent(const double* __restrict
             continue;
         }
         if (active) {
-            const int r = cell_attempt<NS>(c, rtol, atol);
+            const int r = cell::attempt<NS, false, 1>(c, rtol, atol, Lu);
             if (r != CELL_CONTINUE) {
                 my_attempts += c.attempts;
                 double u[NS + 3];
-                if (r == CELL_DONE && cell_end<NS>(c, u)) {
+                if (r == CELL_DONE && cell::finish<NS>(c, u)) {
 #pragma unroll
                     for (int n = 0; n < NS + 3; ++n) trial[n * count + cell] = u[n];
                     fail[cell] = 0;
@@ -248,7 +252,8 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
                            cost, st, &sh[threadIdx.x >> 5][(threadIdx.x & 31) >> 3]);
         }
     }
-    ChemCell<NS> c;
+    cell::Cell<NS> c;
+    double Lu[cell::NQ * cell::NQ];
     int64_t cell = -1;
     bool active = false, drained = false;
     unsigned long long my_attempts = 0;
@@ -268,18 +273,11 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
                         cell = k;
                         double u[NS + 3];
                         load_cell<NS>(U, cs, cell_index ? cell_index[k] : k, u);
-                        const int r = cell_begin_batched<NS>(c, u, dt_cell ? dt_cell[k] : dt, rtol, atol,
-                                                             h_hist ? h_hist[k] : 0.0);
-                        if (r == CELL_CONTINUE) {
+                        if (cell::begin_warm<NS>(c, u, dt_cell ? dt_cell[k] : dt, h_hist ? h_hist[k] : 0.0) ==
+                            CELL_CONTINUE)
                             active = true;
-                        } else if (r == CELL_DONE && cell_end<NS>(c, u)) {
-#pragma unroll
-                            for (int n = 0; n < NS + 3; ++n) trial[n * count + k] = u[n];
-                            fail[k] = 0;
-                            if (cost) cost[k] = 0;
-                        } else {
+                        else
                             report(st, fail, k, CELL_FAIL);
-                        }
                     } else {
                         none = true;
                     }
@@ -292,15 +290,16 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
             continue;
         }
         if (active) {
-            const int r = cell_attempt<NS>(c, rtol, atol);
+            bool screened = false;
+            const int r = cell::attempt<NS, true, 1>(c, rtol, atol, Lu, &screened);
             if (r != CELL_CONTINUE) {
                 my_attempts += c.attempts;
                 double u[NS + 3];
-                if (r == CELL_DONE && cell_end<NS>(c, u)) {
+                if (r == CELL_DONE && cell::finish<NS>(c, u)) {
 #pragma unroll
                     for (int n = 0; n < NS + 3; ++n) trial[n * count + cell] = u[n];
                     fail[cell] = 0;
-                    if (h_hist) h_hist[cell] = c.h;
+                    if (h_hist && !screened) h_hist[cell] = c.h;
                     if (cost) cost[cell] = c.attempts;
                 } else {
                     report(st, fail, cell, r == CELL_MAXSTEPS ? CELL_MAXSTEPS : CELL_FAIL);

@@ -176,38 +176,24 @@ __device__ __noinline__ bool solve_T_slow(const double* w, double et, double& T,
     return true;
 }
 
-// Solves e(T) = R et for the weights w (moles, or with MASS partial densities).  T holds
-// the starting guess on entry (any value) and the converged temperature on exit; m the
-// FP64 mixture coefficients of its range, cv the heat capacity poly_cv(m, T).
+// Solves e(T) = R et for the weights w (moles, or with MASS partial densities): T, the
+// FP64 mixture coefficients m of its range and the heat capacity cv = poly_cv(m, T).  T on
+// entry starts the iteration of states that need solve_T_any.
 //
 // FP64 instructions are what this costs, so one FP64 Newton step of second order replaces
 // the iteration to 1e-10: e(T0) against its values at T_LO, T_MID and T_HI in FP32 picks
-// the range and a secant guess, FP32 Newton steps converge to FP32 accuracy (T within
-// about 1e-6), and with r = et - e(T0) the FP64 step
+// the range and a secant guess t (solve_T_from takes both from its caller), FP32 Newton
+// steps converge to FP32 accuracy (T within about 1e-6), and with r = et - e(T0) the FP64
+// step
 //     T = T0 + d - (cv'/2cv) d^2,  d = r / cv
 // leaves an error of order (d/T)^3, below rounding for d <= 4e-6 T.  The mixture
 // coefficients (a sum over species for each power of T) are most of what is left: 90 FP64
 // instructions a solve.  States near T_mid, outside [T_LO, T_HI], or whose FP32 phase does
 // not settle take solve_T_any.
-template <int NS, bool MASS = false>
-__device__ __forceinline__ bool solve_T(const double* w, double et, double& T, double* m, double& cv) {
-    float t, etf = fp_to_f32(et);
-    bool low;
-    {
-        float lo = 0.0f, mid = 0.0f, hi = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            const float f = fp_to_f32(w[k]);
-            lo = fmaf(f, (float)(MASS ? D_EAT_MASS.lo[k] : D_EAT.lo[k]), lo);
-            mid = fmaf(f, (float)(MASS ? D_EAT_MASS.mid[k] : D_EAT.mid[k]), mid);
-            hi = fmaf(f, (float)(MASS ? D_EAT_MASS.hi[k] : D_EAT.hi[k]), hi);
-        }
-        low = etf <= mid;
-        t = low ? (float)T_LO + (etf - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
-                : (float)TMID + (etf - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
-        const float g = fp_to_f32(T);  // a guess on the same side of T_mid replaces the secant's
-        if (g > 200.0f && g < 6000.0f && (g <= (float)TMID) == low && g != (float)TMID) t = g;
-    }
+template <int NS, bool MASS>
+__device__ __forceinline__ bool solve_T_from(const double* w, double et, bool low, float t, double& T, double* m,
+                                             double& cv) {
+    const float etf = fp_to_f32(et);
     if (low) mix_coef_r<NS, 0, MASS>(w, m);
     else mix_coef_r<NS, 1, MASS>(w, m);
     float mf[6], dt = 0.0f;
@@ -262,6 +248,26 @@ __device__ __forceinline__ bool solve_T(const double* w, double et, double& T, d
     T = Ts;
     cv = cvs;
     return ok;
+}
+template <int NS, bool MASS = false>
+__device__ __forceinline__ bool solve_T(const double* w, double et, double& T, double* m, double& cv) {
+    float t;
+    const float etf = fp_to_f32(et);
+    bool low;
+    {
+        float lo = 0.0f, mid = 0.0f, hi = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            const float f = fp_to_f32(w[k]);
+            lo = fmaf(f, (float)(MASS ? D_EAT_MASS.lo[k] : D_EAT.lo[k]), lo);
+            mid = fmaf(f, (float)(MASS ? D_EAT_MASS.mid[k] : D_EAT.mid[k]), mid);
+            hi = fmaf(f, (float)(MASS ? D_EAT_MASS.hi[k] : D_EAT.hi[k]), hi);
+        }
+        low = etf <= mid;
+        t = low ? (float)T_LO + (etf - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
+                : (float)TMID + (etf - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
+    }
+    return solve_T_from<NS, MASS>(w, et, low, t, T, m, cv);
 }
 
 // The same for a specific energy e (J/kg) and weights z_k = Y_k / W_k, from a warm guess:
@@ -359,6 +365,23 @@ template <int NS>
 __device__ __forceinline__ bool properties(const double* q, Props& s, double T_guess) {
     Prim pr;
     return properties<NS>(q, s, T_guess, pr);
+}
+
+// A temperature of the state q near its own (secants of e(T) in FP32), to start a solve.
+template <int NS>
+__device__ __forceinline__ double estimate_T(const double* q, double et) {
+    float lo = 0.0f, mid = 0.0f, hi = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        const float f = fp_to_f32(q[k]);
+        lo = fmaf(f, (float)D_EAT_MASS.lo[k], lo);
+        mid = fmaf(f, (float)D_EAT_MASS.mid[k], mid);
+        hi = fmaf(f, (float)D_EAT_MASS.hi[k], hi);
+    }
+    const float e = fp_to_f32(et);
+    const float t = e <= mid ? (float)T_LO + (e - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
+                             : (float)TMID + (e - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
+    return t > 50.0f && t < 9000.0f ? fp_from_f32(t) : 1000.0;
 }
 
 // properties<NS>(q, ...) as a yes or no, without FP64 instructions where the answer is

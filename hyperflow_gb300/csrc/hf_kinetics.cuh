@@ -387,16 +387,6 @@ __device__ __forceinline__ void all_jac_rates(const KinCtx<NS>& kc, const double
 }
 
 // ---------------------------------------------------------------- ODE pieces
-template <int NS>
-struct ChemCell {
-    static constexpr int N = NS - 1;
-    double y[N], f0[N], J[N * N];
-    double h, t, tend, rho, e, T, Tsave;
-    double mom[3];  // rho*u, rho*v, rho*E: chemistry leaves them unchanged
-    int steps, attempts;
-    bool rejectLast, rejectMore, needJ;
-};
-
 // composition of y (Y_0..Y_{N-1}; last species closes) -> z = Y/W, C = rho Y/W
 template <int NS>
 __device__ __forceinline__ void comp(const double* y, double rho, double* z, double* C) {
@@ -468,50 +458,6 @@ __device__ __noinline__ bool chem_jac(double rho, double e, double& T, const dou
     return true;
 }
 
-// chem_rhs and chem_jac at the same y from one temperature solve and one pass over
-// the reactions: dy equals chem_rhs's result (same rate arithmetic, same order) and J
-// chem_jac's.
-template <int NS>
-__device__ __noinline__ bool chem_rhs_jac(double rho, double e, double& T, const double* y, double* dy, double* J) {
-    constexpr int N = NS - 1, L = NS - 1;
-    double z[NS], C[NS], m[6];
-    comp<NS>(y, rho, z, C);
-    double Tn = T;
-    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
-    T = Tn;
-    KinCtx<NS> kc;
-    kin_setup<NS>(T, C, kc);
-    double JC[N * NS], JT[N], w[NS];
-#pragma unroll
-    for (int i = 0; i < N * NS; ++i) JC[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) JT[i] = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) w[k] = 0.0;
-    all_jac_rates<NS>(kc, C, JC, JT, w, std::make_index_sequence<NR>{});
-    bool ok = true;
-    const double ir = 1.0 / rho;
-#pragma unroll
-    for (int k = 0; k < NS - 1; ++k) {
-        dy[k] = w[k] * D_MW.v[k] * ir;
-        ok = ok && isfinite(dy[k]);
-    }
-    if (!ok) return false;
-    const double cv = poly_cv(m, T);
-    double dTdy[N];
-    const double eL = (kc.hRT[L] - 1.0) * INVW.v[L];
-#pragma unroll
-    for (int j = 0; j < N; ++j) dTdy[j] = -T * ((kc.hRT[j] - 1.0) * INVW.v[j] - eL) / cv;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const double cl = JC[i * NS + L] * INVW.v[L];
-        const double ti = JT[i] * ir;
-#pragma unroll
-        for (int j = 0; j < N; ++j) J[i * N + j] = D_MW.v[i] * (JC[i * NS + j] * INVW.v[j] - cl + ti * dTdy[j]);
-    }
-    return true;
-}
-
 // ---------------------------------------------------------------- Rodas4
 __device__ constexpr double RA[15] = {
     1.544, 0.9466785280815826, 0.2557011698983284, 3.314825187068521, 2.896124015972201,
@@ -528,18 +474,6 @@ constexpr double RGAMMA = 0.25;
 constexpr long MAX_STEPS = 5000;
 
 enum : int { CELL_CONTINUE = 0, CELL_DONE = 1, CELL_FAIL = 2, CELL_MAXSTEPS = 3 };
-
-template <int N>
-__device__ __forceinline__ double wrms(const double* v, const double* y0, const double* y1, double rtol, double atol) {
-    double s = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const double sc = atol + rtol * fmax(fabs(y0[i]), fabs(y1[i]));
-        const double r = v[i] / sc;
-        s = fma(r, r, s);
-    }
-    return fmax(sqrt(s * (1.0 / N)), 1e-10);
-}
 
 // LU with partial pivoting in place (P A = L U); the diagonal holds 1/U_kk.
 template <int N>
@@ -583,279 +517,6 @@ __device__ __forceinline__ void lu_solve(const double* A, const int* piv, double
         for (int j = i + 1; j < N; ++j) b[i] = fma(-A[i * N + j], b[j], b[i]);
         b[i] *= A[i * N + i];  // reciprocal pivot
     }
-}
-
-// Loads a cell and prepares the integration (chemistry.cpp:55-62 + the starting
-// step of the integrator).  Returns CELL_CONTINUE or CELL_FAIL.
-template <int NS>
-__device__ __noinline__ int cell_begin(ChemCell<NS>& c, const double* u, double dt, double rtol, double atol) {
-    constexpr int N = NS - 1;
-    if (!(dt > 0.0) || !isfinite(dt)) return CELL_FAIL;
-    Props pr;
-    if (!properties<NS>(u, pr, 1000.0)) return CELL_FAIL;
-    double rho = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) rho += u[k];
-    const double ir = 1.0 / rho;
-    const double uu = u[NS] * ir, vv = u[NS + 1] * ir;
-    c.rho = rho;
-    c.e = u[NS + 2] * ir - 0.5 * (uu * uu + vv * vv);
-    c.mom[0] = u[NS];
-    c.mom[1] = u[NS + 1];
-    c.mom[2] = u[NS + 2];
-    c.T = pr.T;
-#pragma unroll
-    for (int k = 0; k < N; ++k) c.y[k] = u[k] * ir;
-    // f0 and the first step's Jacobian
-    if (!chem_rhs_jac<NS>(c.rho, c.e, c.T, c.y, c.f0, c.J)) return CELL_FAIL;
-    c.Tsave = c.T;
-    // starting step: Hairer's estimate in time scaled by the interval
-    {
-        const double Ts = c.T;
-        const double d0 = wrms<N>(c.y, c.y, c.y, rtol, atol), d1 = wrms<N>(c.f0, c.y, c.y, rtol, atol) * dt;
-        const double hh = d1 < 1e-5 ? 1.0 : fmin(1.0, 0.01 * d0 / d1);
-        double yn[N], fy[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) yn[i] = c.y[i] + hh * dt * c.f0[i];
-        double d2;
-        if (chem_rhs<NS>(c.rho, c.e, c.T, yn, fy)) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) fy[i] = (fy[i] - c.f0[i]) / hh;
-            d2 = wrms<N>(fy, c.y, c.y, rtol, atol);
-        } else {
-            d2 = 1e30;
-        }
-        c.T = Ts;
-        const double mx = fmax(d1, d2);
-        const double h1 = mx <= 1e-15 ? 1.0 : pow(0.01 / mx, 0.2);
-        c.h = fmin(fmin(100.0 * hh, h1), 1.0) * dt;
-    }
-    c.h = fmin(c.h, dt);
-    c.t = 0.0;
-    c.tend = dt;
-    c.steps = 0;
-    c.attempts = 0;
-    c.rejectLast = c.rejectMore = false;
-    c.needJ = false;
-    return CELL_CONTINUE;
-}
-
-// One step attempt (the body of the KPP accept loop).
-template <int NS>
-__device__ __noinline__ int cell_attempt(ChemCell<NS>& c, double rtol, double atol) {
-    constexpr int N = NS - 1;
-    if (c.needJ) {
-        if (c.steps >= MAX_STEPS) return CELL_MAXSTEPS;
-        if (!chem_jac<NS>(c.rho, c.e, c.T, c.y, c.J)) return CELL_FAIL;
-        c.Tsave = c.T;
-        c.needJ = false;
-    }
-    if (++c.attempts > 4 * MAX_STEPS) return CELL_MAXSTEPS;
-    bool last = false;
-    if (c.t + 1.01 * c.h >= c.tend) { c.h = c.tend - c.t; last = true; }
-    double Mx[N * N], K[6][N], yn[N], fy[N];
-    int piv[N];
-    const double inv = 1.0 / (c.h * RGAMMA);
-#pragma unroll
-    for (int i = 0; i < N * N; ++i) Mx[i] = -c.J[i];
-#pragma unroll
-    for (int i = 0; i < N; ++i) Mx[i * N + i] += inv;
-    bool ok = lu_factor<N>(Mx, piv);
-    const double ih = 1.0 / c.h;
-#pragma unroll 1
-    for (int s = 0; s < 6; ++s) {
-        if (!ok) break;
-        const int base = s * (s - 1) / 2;
-        if (s == 0) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) fy[i] = c.f0[i];
-        } else {
-#pragma unroll
-            for (int i = 0; i < N; ++i) {
-                double v = c.y[i];
-#pragma unroll
-                for (int j = 0; j < s; ++j) v = fma(RA[base + j], K[j][i], v);
-                yn[i] = v;
-            }
-            ok = chem_rhs<NS>(c.rho, c.e, c.T, yn, fy);
-            if (!ok) break;
-        }
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            double v = fy[i];
-#pragma unroll
-            for (int j = 0; j < s; ++j) v = fma(RC[base + j] * ih, K[j][i], v);
-            K[s][i] = v;
-        }
-        lu_solve<N>(Mx, piv, K[s]);
-    }
-    double err = __longlong_as_double(0x7ff0000000000000ll);  // +inf
-    if (ok) {
-        double ev[N];
-        bool fin = true;
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            double v = c.y[i];
-#pragma unroll
-            for (int s = 0; s < 6; ++s) v = fma(RM[s], K[s][i], v);
-            yn[i] = v;
-            ev[i] = K[5][i];
-            fin = fin && isfinite(v);
-        }
-        err = wrms<N>(ev, c.y, yn, rtol, atol);
-        if (!fin) err = __longlong_as_double(0x7ff0000000000000ll);
-    }
-    if (!isfinite(err)) {
-        c.T = c.Tsave;
-        c.h *= 0.25;
-        c.rejectLast = true;
-        if (!(c.h > 1e-300) || c.t + c.h == c.t) return CELL_FAIL;
-        return CELL_CONTINUE;
-    }
-    double hnew = c.h * fmin(6.0, fmax(0.2, 0.9 / sqrt(sqrt(err))));
-    if (err <= 1.0) {
-        c.t = last ? c.tend : c.t + c.h;
-#pragma unroll
-        for (int i = 0; i < N; ++i) c.y[i] = yn[i];
-        if (c.rejectLast) hnew = fmin(hnew, c.h);
-        c.rejectLast = c.rejectMore = false;
-        ++c.steps;
-        c.h = hnew;
-        if (!(c.t < c.tend)) return CELL_DONE;
-        if (c.steps >= MAX_STEPS) return CELL_MAXSTEPS;
-        // f0 and the next step's Jacobian at the new y
-        if (!chem_rhs_jac<NS>(c.rho, c.e, c.T, c.y, c.f0, c.J)) return CELL_FAIL;
-        c.Tsave = c.T;
-        return CELL_CONTINUE;
-    }
-    if (c.rejectMore) hnew = c.h * 0.1;
-    c.rejectMore = c.rejectLast;
-    c.rejectLast = true;
-    c.T = c.Tsave;
-    c.h = hnew;
-    if (!(c.h > 1e-300) || c.t + c.h == c.t) return CELL_FAIL;
-    return CELL_CONTINUE;
-}
-
-// chemistry.cpp:63-70: clip, close the mass with the last species, final check.
-// Writes the whole state u (momentum and energy as they came in).
-template <int NS>
-__device__ __noinline__ bool cell_end(const ChemCell<NS>& c, double* u) {
-    constexpr int N = NS - 1;
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        const double v = c.y[k];
-        if (!isfinite(v) || v < -1e-13) return false;
-        u[k] = c.rho * fmax(0.0, v);
-        s += u[k];
-    }
-    u[N] = c.rho - s;
-    u[NS] = c.mom[0];
-    u[NS + 1] = c.mom[1];
-    u[NS + 2] = c.mom[2];
-    Props pr;
-    return properties<NS>(u, pr, c.T);
-}
-
-// ---------------------------------------------------------------- batched form
-// Batched-form start of a cell (extension to the reference's per-call CVODE
-// restart).  After f0 = f(y0) and J = df/dy at y0:
-//  * frozen-cell screen: in the scaled variables z_i = y_i / sc_i
-//    (sc_i = atol + rtol |y_i|), with a = ||J_z||_inf dt, if a <= 20,
-//    ||f0_z||_inf dt e^a <= 1 and ||f0_z||_inf dt a^2 e^a / 6 <= 1e-5, the interval
-//    is taken as one second-order Taylor step y1 = y0 + dt f0 + dt^2/2 J f0: for the
-//    linearised system its remainder sum_{k>=3} dt^k/k! J^(k-1) f0 is bounded by
-//    the last expression, i.e. below 1e-5 tolerance units;
-//  * otherwise the first step size is the cell's proposed step from the previous
-//    call (h_prev > 0), else the same starting-step estimate as cell_begin; the
-//    Jacobian just formed is the first step's Jacobian.
-// Returns CELL_DONE (screened), CELL_CONTINUE or CELL_FAIL.
-template <int NS>
-__device__ __noinline__ int cell_begin_batched(ChemCell<NS>& c, const double* u, double dt, double rtol, double atol,
-                                               double h_prev) {
-    constexpr int N = NS - 1;
-    if (!(dt > 0.0) || !isfinite(dt)) return CELL_FAIL;
-    Props pr;
-    if (!properties<NS>(u, pr, 1000.0)) return CELL_FAIL;
-    double rho = 0.0;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) rho += u[k];
-    const double ir = 1.0 / rho;
-    const double uu = u[NS] * ir, vv = u[NS + 1] * ir;
-    c.rho = rho;
-    c.e = u[NS + 2] * ir - 0.5 * (uu * uu + vv * vv);
-    c.mom[0] = u[NS];
-    c.mom[1] = u[NS + 1];
-    c.mom[2] = u[NS + 2];
-    c.T = pr.T;
-#pragma unroll
-    for (int k = 0; k < N; ++k) c.y[k] = u[k] * ir;
-    if (!chem_rhs_jac<NS>(c.rho, c.e, c.T, c.y, c.f0, c.J)) return CELL_FAIL;
-    c.Tsave = c.T;
-    c.t = 0.0;
-    c.tend = dt;
-    c.steps = 0;
-    c.attempts = 0;
-    c.rejectLast = c.rejectMore = false;
-    c.needJ = false;
-    double sc[N], fz = 0.0, jz = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        sc[i] = atol + rtol * fabs(c.y[i]);
-        fz = fmax(fz, fabs(c.f0[i]) / sc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        double r = 0.0;
-#pragma unroll
-        for (int j = 0; j < N; ++j) r = fma(fabs(c.J[i * N + j]), sc[j], r);
-        jz = fmax(jz, r / sc[i]);
-    }
-    // remainder of the second-order Taylor step for the linearised system:
-    // ||R||_z <= fz dt * a^2 e^a / 6 with a = jz dt; the whole change stays below
-    // fz dt e^a <= 1 tolerance unit, so J is constant over the interval to far
-    // better than the tolerance
-    const double a = jz * dt;
-    const double ea = a <= 20.0 ? exp(a) : 1e300;
-    if (a <= 20.0 && fz * dt * ea <= 1.0 && fz * dt * a * a * ea <= 6e-5) {
-        double jf[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) {
-            double v = 0.0;
-#pragma unroll
-            for (int j = 0; j < N; ++j) v = fma(c.J[i * N + j], c.f0[j], v);
-            jf[i] = v;
-        }
-#pragma unroll
-        for (int i = 0; i < N; ++i) c.y[i] = fma(0.5 * dt * dt, jf[i], fma(dt, c.f0[i], c.y[i]));
-        c.t = dt;
-        c.h = dt;
-        return CELL_DONE;
-    }
-    if (h_prev > 0.0 && isfinite(h_prev)) {
-        c.h = fmin(h_prev, dt);
-    } else {
-        const double Ts = c.T;
-        const double d0 = wrms<N>(c.y, c.y, c.y, rtol, atol), d1 = wrms<N>(c.f0, c.y, c.y, rtol, atol) * dt;
-        const double hh = d1 < 1e-5 ? 1.0 : fmin(1.0, 0.01 * d0 / d1);
-        double yn[N], fy[N];
-#pragma unroll
-        for (int i = 0; i < N; ++i) yn[i] = c.y[i] + hh * dt * c.f0[i];
-        double d2;
-        if (chem_rhs<NS>(c.rho, c.e, c.T, yn, fy)) {
-#pragma unroll
-            for (int i = 0; i < N; ++i) fy[i] = (fy[i] - c.f0[i]) / hh;
-            d2 = wrms<N>(fy, c.y, c.y, rtol, atol);
-        } else {
-            d2 = 1e30;
-        }
-        c.T = Ts;
-        const double mx = fmax(d1, d2);
-        const double h1 = mx <= 1e-15 ? 1.0 : pow(0.01 / mx, 0.2);
-        c.h = fmin(fmin(100.0 * hh, h1), 1.0) * dt;
-    }
-    return CELL_CONTINUE;
 }
 
 }  // namespace hf
