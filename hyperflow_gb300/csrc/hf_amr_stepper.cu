@@ -515,7 +515,7 @@ cudaError_t g_react(hf_amr* m, double* const* X, cudaStream_t s, int64_t* nl) {
     for (int l = 0; e == cudaSuccess && l <= m->finest; ++l) {
         AmrLevel& a = m->lev[l];
         if (!a.nleaf) continue;
-        e = cudaMemsetAsync(&m->gst->counter, 0, 2 * sizeof(unsigned long long), s);  // work-queue heads
+        e = cudaMemsetAsync(&m->gst->counter, 0, 3 * sizeof(unsigned long long), s);  // work-queue heads
         if (e == cudaSuccess)
             e = hf::launch_chem_batched(m->ns, X[l], a.dom.comp_stride, a.cells, a.nleaf, 0.0, m->ddt, nullptr,
                                         m->o.rtol, m->o.atol, a.hist.h, a.hist.cost, a.order, a.bins, a.trial, a.fail,

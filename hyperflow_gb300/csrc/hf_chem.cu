@@ -17,10 +17,11 @@
 // reaction structure, temperature exponents and activation temperatures are
 // compile-time constants of the generated mechanism table, so every species index
 // is a register index.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include "hf_cell.cuh"
-#include "hf_chem_coop.cuh"
+#include "hf_group.cuh"
 
 namespace hf {
 
@@ -142,93 +143,112 @@ __global__ void k_chem_commit(double* __restrict__ U, int64_t cs, const int64_t*
     for (int n = 0; n < NS + 3; ++n) U[b + n * cs] = trial[n * count + i];
 }
 
-// Batched form: the persistent lane-refill loop of k_chem_persistent over a work
-// queue ordered most-expensive-first (order[]), starting each cell with
-// cell_begin_batched, and recording per cell the attempts taken (cost[]) and the
-// controller's proposed next step (h_hist[]) for the next call.
-// Cooperative phase of the batched kernel: queue positions [0, ncoop) (the costliest
-// buckets), one cell per group of 8 lanes (hf_chem_coop.cuh), the refill scheme of the
-// per-lane loop with groups in place of lanes.
-template <int NS>
-__device__ __forceinline__ void coop_phase(const double* __restrict__ U, int64_t cs,
-                                           const int64_t* __restrict__ cell_index, const int32_t* __restrict__ order,
-                                           int64_t count, int64_t ncoop, double dt, const double* __restrict__ dt_cell,
-                                           double rtol, double atol, double* __restrict__ trial,
-                                           int* __restrict__ fail, double* __restrict__ h_hist,
-                                           int32_t* __restrict__ cost, DevStatus* st, coop::GShared* sh) {
-    using namespace coop;
-    const Grp g = grp();
+// Cells of a queue (positions [0, n) of order, or cells 0..n-1), one per group of 8 lanes
+// (hf_group.cuh): the refill scheme of the per-lane loop with groups in place of lanes.
+// Returns the step attempts of the caller's cells (on the first lane of each group).
+template <int NS, bool SCREEN>
+__device__ __forceinline__ unsigned long long group_phase(const double* __restrict__ U, int64_t cs,
+                                                          const int64_t* __restrict__ cell_index,
+                                                          const int32_t* __restrict__ order, int64_t n, int64_t count,
+                                                          double dt, const double* __restrict__ dt_cell, double rtol,
+                                                          double atol, double* __restrict__ trial,
+                                                          int* __restrict__ fail, double* __restrict__ h_hist,
+                                                          int32_t* __restrict__ cost, DevStatus* st,
+                                                          grp8::Shared* sh) {
     const unsigned lane = threadIdx.x & 31;
-    GInt c{};
-    double y = 0.0, f0 = 0.0, J[NQ];
-#pragma unroll
-    for (int j = 0; j < NQ; ++j) J[j] = 0.0;
+    const int t = grp8::lane8();
+    grp8::Cell<NS> c;
+    c.active = false;
     int64_t cell = -1;
-    bool active = false, drained = false;
-    unsigned long long my_attempts = 0;
-    auto finish = [&](int64_t k, bool screened) {
-        double u[NS + 3];
-        const bool ok = gend<NS>(g, c, y, u, sh->T);
-        if (g.t == 0) {
-            if (ok) {
-#pragma unroll
-                for (int n = 0; n < NS + 3; ++n) trial[n * count + k] = u[n];
-                fail[k] = 0;
-                if (!screened && h_hist) h_hist[k] = c.h;
-                if (cost) cost[k] = screened ? 0 : c.attempts;
-            } else {
-                report(st, fail, k, CELL_FAIL);
-            }
-        }
-    };
+    bool drained = false, loaded = false;
+    unsigned long long attempts = 0;
     for (;;) {
         if (!drained) {
-            const unsigned need = __ballot_sync(0xffffffffu, !active) & 0x01010101u;  // first lane of each group
+            const unsigned need = __ballot_sync(0xffffffffu, !c.active) & 0x01010101u;  // first lane of each group
             bool none = false;
             if (need) {
                 const int leader = __ffs(need) - 1;
                 unsigned long long base = 0;
                 if ((int)lane == leader) base = atomicAdd(&st->coop_counter, (unsigned long long)__popc(need));
                 base = __shfl_sync(0xffffffffu, base, leader);
-                if (!active) {
-                    const int64_t q = (int64_t)(base + __popc(need & ((1u << g.base) - 1u)));
-                    if (q < ncoop) {
-                        const int64_t k = (int64_t)order[q];
-                        cell = k;
+                if (!c.active) {
+                    const int64_t q = (int64_t)(base + __popc(need & ((1u << (lane & 24)) - 1u)));
+                    const bool got = q < n;
+                    none = !got;
+                    // a group that never held a cell computes along on the queue's first one
+                    if (got || !loaded) {
+                        const int64_t p = got ? q : 0, k = order ? (int64_t)order[p] : p;
                         double u[NS + 3];
-                        const int64_t b = cell_index ? cell_index[k] : k;
-#pragma unroll
-                        for (int n = 0; n < NS + 3; ++n) u[n] = U[b + n * cs];
-                        const int r = gbegin<NS>(g, c, y, f0, J, u, dt_cell ? dt_cell[k] : dt, rtol, atol,
-                                                 h_hist ? h_hist[k] : 0.0, sh);
-                        if (g.t == 0) atomicAdd(&st->coop_cells, 1ull);
-                        if (r == CELL_CONTINUE) active = true;
-                        else if (r == CELL_DONE) finish(k, true);
-                        else if (g.t == 0) report(st, fail, k, CELL_FAIL);
-                    } else {
-                        none = true;
+                        load_cell<NS>(U, cs, cell_index ? cell_index[k] : k, u);
+                        const bool ok = grp8::load<NS>(c, u, dt_cell ? dt_cell[k] : dt, h_hist ? h_hist[k] : 0.0);
+                        loaded = true;
+                        if (got) {
+                            cell = k;
+                            c.active = ok;
+                            if (t == 0 && SCREEN) atomicAdd(&st->coop_cells, 1ull);
+                            if (t == 0 && !ok) report(st, fail, k, CELL_FAIL);
+                        }
                     }
                 }
             }
             drained = __any_sync(0xffffffffu, none);
         }
-        if (!__any_sync(0xffffffffu, active)) {
+        if (!__any_sync(0xffffffffu, c.active)) {
             if (drained) break;
             continue;
         }
-        if (active) {
-            const int r = gattempt<NS>(g, c, y, f0, J, rtol, atol, sh);
-            if (r != CELL_CONTINUE) {
-                if (g.t == 0) my_attempts += c.attempts;
-                if (r == CELL_DONE) finish(cell, false);
-                else if (g.t == 0) report(st, fail, cell, r == CELL_MAXSTEPS ? CELL_MAXSTEPS : CELL_FAIL);
-                active = false;
+        bool screened = false;
+        const int r = grp8::attempt<NS, SCREEN>(c, rtol, atol, sh, screened);
+        const bool done = c.active && r != CELL_CONTINUE;
+        if (__any_sync(0xffffffffu, done)) {
+            double u[NS + 3];
+            const bool keep = grp8::finish<NS>(c, u);
+            if (done) {
+                if (t == 0) attempts += c.attempts;
+                if (r == CELL_DONE && keep) {
+#pragma unroll
+                    for (int m = 0; m < NS + 3; ++m)
+                        if ((m & 7) == t) trial[m * count + cell] = u[m];
+                    if (t == 0) {
+                        fail[cell] = 0;
+                        if (h_hist && !screened) h_hist[cell] = c.h;
+                        if (cost) cost[cell] = c.attempts;
+                    }
+                } else if (t == 0) {
+                    report(st, fail, cell, r == CELL_MAXSTEPS ? CELL_MAXSTEPS : CELL_FAIL);
+                }
+                c.active = false;
             }
         }
     }
-    if (my_attempts) atomicAdd(&st->steps, my_attempts);
+    return attempts;
 }
 
+// The plain and persistent forms of a small batch: every cell in a group.
+template <int NS>
+__global__ void __launch_bounds__(64) k_chem_group(const double* __restrict__ U, int64_t cs,
+                                                   const int64_t* __restrict__ cell_index, int64_t count, double dt,
+                                                   const double* __restrict__ dt_dev,
+                                                   const double* __restrict__ dt_cell, double rtol, double atol,
+                                                   double* __restrict__ trial, int* __restrict__ fail, DevStatus* st) {
+    __shared__ grp8::Shared sh[8];
+    if (st->abort_run) return;
+    if (dt_dev) dt = *dt_dev;
+    const unsigned long long a =
+        group_phase<NS, false>(U, cs, cell_index, nullptr, count, count, dt, dt_cell, rtol, atol, trial, fail, nullptr,
+                               nullptr, st, &sh[threadIdx.x >> 3]);
+    if (a) atomicAdd(&st->steps, a);
+}
+
+// Measured on the batched form (warm history): 65,536 cells of very uneven stiffness 351 ms
+// without groups, 141 with them (4,639 cells of 255 to 1,340 attempts); 512 x 128 cells with
+// 19,400 burning ones 80 ms in order of arrival, 49 with one warp of them to a
+// sub-partition; 1D detonation of 4,000 cells 149 ms (8 steps) on lanes, 58 with groups.
+//
+// Batched form: the persistent lane-refill loop of k_chem_persistent over a work
+// queue ordered most-expensive-first (order[]), starting each cell with
+// cell_begin_batched, and recording per cell the attempts taken (cost[]) and the
+// controller's proposed next step (h_hist[]) for the next call.
 template <int NS, int MINB, bool COOP>
 __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restrict__ U, int64_t cs,
                                                      const int64_t* __restrict__ cell_index,
@@ -237,26 +257,36 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
                                                      const double* __restrict__ dt_cell, double rtol, double atol,
                                                      double* __restrict__ trial, int* __restrict__ fail,
                                                      double* __restrict__ h_hist, int32_t* __restrict__ cost,
-                                                     const unsigned long long* __restrict__ coop_n, DevStatus* st) {
+                                                     const unsigned long long* __restrict__ coop_n, int64_t lanes_first,
+                                                     DevStatus* st) {
     if (st->abort_run) return;  // an earlier step of this device-resident run failed
     const unsigned lane = threadIdx.x & 31;
     if (dt_dev) dt = *dt_dev;  // interval from device memory (graph-captured steps)
     // COOP: the costliest cells first, one cell per group of 8 lanes; the rest one per
     // lane.  Without it the kernel holds no shared memory (the L1 keeps the lanes' stacks).
     int64_t ncoop = 0;
+    unsigned long long my_attempts = 0;
     if constexpr (COOP) {
+        __shared__ grp8::Shared sh[8];
         ncoop = (order && coop_n) ? (int64_t)*coop_n : 0;
-        if (ncoop > 0) {
-            __shared__ coop::GShared sh[2][4];  // 64-thread blocks: 2 warps of 4 groups
-            coop_phase<NS>(U, cs, cell_index, order, count, ncoop, dt, dt_cell, rtol, atol, trial, fail, h_hist,
-                           cost, st, &sh[threadIdx.x >> 5][(threadIdx.x & 31) >> 3]);
-        }
+        if (ncoop > 0)
+            my_attempts = group_phase<NS, true>(U, cs, cell_index, order, ncoop, count, dt, dt_cell, rtol, atol, trial,
+                                                fail, h_hist, cost, st, &sh[threadIdx.x >> 3]);
     }
+    // Two queues: the costly cells after the cooperative ones, then the rest.  Warps in the
+    // first slot of their SM sub-partition start with the costly ones and the others with the
+    // rest, so that every sub-partition gets one warp of long step chains before any gets
+    // two (a second one beside it halves both: 244 against 401 us an attempt); when there are
+    // more costly cells than those warps have lanes, all warps start with them.
+    const int64_t nhi = (order && coop_n) ? (int64_t)coop_n[1] : 0;
+    unsigned slot;
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
+    bool costly = nhi > 0 && (slot < 4 || nhi > lanes_first);
+    int dry = 0;  // queues found empty
     cell::Cell<NS> c;
     double Lu[cell::NQ * cell::NQ];
     int64_t cell = -1;
     bool active = false, drained = false;
-    unsigned long long my_attempts = 0;
     for (;;) {
         if (!drained) {
             const unsigned need = __ballot_sync(0xffffffffu, !active);
@@ -264,11 +294,12 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
             if (need) {
                 const int leader = __ffs(need) - 1;
                 unsigned long long base = 0;
-                if ((int)lane == leader) base = atomicAdd(&st->counter, (unsigned long long)__popc(need));
+                if ((int)lane == leader)
+                    base = atomicAdd(costly ? &st->costly_counter : &st->counter, (unsigned long long)__popc(need));
                 base = __shfl_sync(0xffffffffu, base, leader);
                 if (!active) {
-                    const int64_t q = ncoop + (int64_t)(base + __popc(need & ((1u << lane) - 1u)));
-                    if (q < count) {
+                    const int64_t q = ncoop + (costly ? 0 : nhi) + (int64_t)(base + __popc(need & ((1u << lane) - 1u)));
+                    if (q < (costly ? ncoop + nhi : count)) {
                         const int64_t k = order ? (int64_t)order[q] : q;
                         cell = k;
                         double u[NS + 3];
@@ -283,7 +314,10 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
                     }
                 }
             }
-            drained = __any_sync(0xffffffffu, none);
+            if (__any_sync(0xffffffffu, none)) {  // this queue is empty: the other one next
+                costly = !costly;
+                drained = ++dry == 2 || (nhi == 0 && dry == 1);
+            }
         }
         if (!__any_sync(0xffffffffu, active)) {
             if (drained) break;
@@ -316,8 +350,10 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
 //  * blocks of 64 lanes per SM the queue kernel's register budget is built for: 4 (255
 //    registers) or 5, 6, 8 (fewer registers, more resident lanes); the same per-cell code;
 //  * the cooperative queue takes cells that used at least 2^coop_min - 1 attempts in the
-//    previous call (coop_min = NBUCKET, the default: no cooperative phase, and the kernel
+//    previous call (coop_min = NBUCKET: no cooperative phase, and the kernel
 //    instance without it).
+//    COOP_AUTO, the default: k_order_scan decides.
+constexpr int COOP_AUTO = 17;
 std::atomic<int> g_tune_minb{0}, g_tune_coop{0};
 void chem_tuning(int* minb, int* coop_min) {
     if (g_tune_minb.load() == 0) {
@@ -329,8 +365,8 @@ void chem_tuning(int* minb, int* coop_min) {
     if (g_tune_coop.load() == 0) {
         const char* off = getenv("HF_COOP");
         const char* e = getenv("HF_COOP_MIN_BUCKET");
-        int v = e ? atoi(e) : 16;
-        v = v < 1 ? 1 : (v > 16 ? 16 : v);
+        int v = e ? atoi(e) : COOP_AUTO;
+        if (e) v = v < 1 ? 1 : (v > COOP_AUTO ? 16 : v);
         if (off && atoi(off) == 0) v = 16;
         int expect = 0;
         g_tune_coop.compare_exchange_strong(expect, v);
@@ -342,40 +378,87 @@ void chem_tuning(int* minb, int* coop_min) {
 // Work-queue order: counting sort of cells by bucket = floor(log2(cost + 1)) (16
 // buckets), most expensive bucket first.  Cells of one bucket keep no particular
 // order; each cell's result does not depend on its position.
-constexpr int NBUCKET = 16;
-__device__ __forceinline__ int cost_bucket(int32_t c) {
-    const int b = 31 - __clz((unsigned)c + 1u);
-    return min(b, NBUCKET - 1);
+// With SUB sub-buckets to a factor of two the cells of a warp have about the same cost.
+constexpr int NBUCKET = 16, SUB = 8, NBIN = NBUCKET * SUB;
+constexpr int COSTLY_BUCKET = 4;  // at least 15 attempts
+static_assert(NBIN + 2 <= CHEM_BINS, "bins");
+__device__ __forceinline__ int cost_bin(int32_t c) {
+    const unsigned m = (unsigned)c + 1u;
+    const int b = 31 - __clz(m);
+    return min(b * SUB + (int)(((unsigned long long)m * SUB >> b) - SUB), NBIN - 1);
 }
 __global__ void k_order_hist(const int32_t* __restrict__ cost, int64_t count, unsigned long long* __restrict__ bins) {
-    __shared__ unsigned int sb[NBUCKET];
-    if (threadIdx.x < NBUCKET) sb[threadIdx.x] = 0;
+    __shared__ unsigned int sb[NBIN];
+    if (threadIdx.x < NBIN) sb[threadIdx.x] = 0;
     __syncthreads();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(&sb[cost_bucket(max(cost[i], 0))], 1u);
+        atomicAdd(&sb[cost_bin(max(cost[i], 0))], 1u);
     __syncthreads();
-    if (threadIdx.x < NBUCKET && sb[threadIdx.x]) atomicAdd(&bins[threadIdx.x], (unsigned long long)sb[threadIdx.x]);
+    if (threadIdx.x < NBIN && sb[threadIdx.x]) atomicAdd(&bins[threadIdx.x], (unsigned long long)sb[threadIdx.x]);
 }
-// bins[b] -> start offset of bucket b, descending buckets first; bins[NBUCKET] = the
-// cells of the cooperative queue: whole buckets from the costliest down to min_bucket
-// while they fit in cap cells (whole buckets, so the choice does not depend on the
-// order within a bucket).
-__global__ void k_order_scan(unsigned long long* bins, unsigned long long cap, int min_bucket) {
-    unsigned long long off = 0, ncoop = 0;
+// bins[b] -> start offset of bin b, descending bins first; bins[NBIN] = the cells of the
+// cooperative queue: whole bins from the costliest down to bucket min_bucket while they fit
+// in cap cells (whole bins, so the choice does not depend on the order within one);
+// bins[NBIN + 1] = the cells after them in buckets from COSTLY_BUCKET up.
+// min_bucket < 0: the line with the least estimated time, the root of the sum of squares
+// (they run side by side, but slow each other) of
+//   the FP64 pipe's:  attempts of the groups / 33.8 + attempts of the lanes / 97 per us,
+//   the longest chain in a group:  73 us an attempt alone, 113 beside a second warp,
+//   the longest chain on a lane:   244 us an attempt with one warp of costly cells to a
+//                                  sub-partition and no groups, 401 beside another warp
+// (measured, 10 species, cells of 398 attempts, 152 SMs).  A group's chain is three times
+// as fast and costs the pipe three times as much: it pays for cells far above the mean.
+constexpr float GROUP_RATE = 33.8f, LANE_RATE = 97.0f, GROUP_ALONE = 73.0f, GROUP_PAIR = 113.0f, LANE_ALONE = 244.0f,
+                LANE_PAIR = 401.0f;
+__device__ __forceinline__ float bin_cost(int b) {  // attempts at the bin's lower edge
+    return (float)(1u << (b / SUB)) * (1.0f + (float)(b % SUB) / SUB) - 1.0f;
+}
+__global__ void k_order_scan(unsigned long long* bins, unsigned long long cap, int min_bucket, int subparts) {
+    int min_bin = min_bucket * SUB;
+    if (min_bucket < 0) {
+        float total = 0.0f, most = 0.0f;
+        unsigned long long costly = 0;
+        for (int b = 0; b < NBIN; ++b) {
+            total += (float)bins[b] * bin_cost(b);
+            if (bins[b]) most = bin_cost(b + 1);
+            if (b >= COSTLY_BUCKET * SUB) costly += bins[b];
+        }
+        const float r = 608.0f / (float)subparts;
+        min_bin = NBIN;
+        const float p0 = total / LANE_RATE * r, l0 = most * (costly <= 32ull * subparts ? LANE_ALONE : LANE_PAIR);
+        float best = p0 * p0 + l0 * l0;
+        float grp = 0.0f;
+        unsigned long long n = 0;
+        for (int b = NBIN - 1; b >= 3 * SUB; --b) {
+            n += bins[b];
+            if (n > cap) break;
+            grp += (float)bins[b] * bin_cost(b);
+            const float p = (grp / GROUP_RATE + (total - grp) / LANE_RATE) * r;
+            const float g = most * (n <= 4ull * subparts ? GROUP_ALONE : GROUP_PAIR), l = bin_cost(b) * LANE_PAIR;
+            const float t = p * p + g * g + l * l;
+            if (bins[b] && t < best) {
+                best = t;
+                min_bin = b;
+            }
+        }
+    }
+    unsigned long long off = 0, ncoop = 0, costly = 0;
     bool open = true;
-    for (int b = NBUCKET - 1; b >= 0; --b) {
+    for (int b = NBIN - 1; b >= 0; --b) {
         const unsigned long long n = bins[b];
-        if (open && b >= min_bucket && ncoop + n <= cap) ncoop += n;
+        if (open && b >= min_bin && ncoop + n <= cap) ncoop += n;
         else open = false;
+        if (!open && b >= COSTLY_BUCKET * SUB) costly += n;
         bins[b] = off;
         off += n;
     }
-    bins[NBUCKET] = ncoop;
+    bins[NBIN] = ncoop;
+    bins[NBIN + 1] = costly;
 }
 __global__ void k_order_scatter(const int32_t* __restrict__ cost, int64_t count, unsigned long long* __restrict__ bins,
                                 int32_t* __restrict__ order) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long pos = atomicAdd(&bins[cost_bucket(max(cost[i], 0))], 1ull);
+        const unsigned long long pos = atomicAdd(&bins[cost_bin(max(cost[i], 0))], 1ull);
         order[pos] = (int32_t)i;
     }
 }
@@ -388,7 +471,7 @@ static cudaError_t chem_batched_impl(double* U, int64_t cs, const int64_t* idx, 
                                      int64_t* launches) {
     int minb, coop_min;
     chem_tuning(&minb, &coop_min);
-    const bool coop = coop_min < NBUCKET;
+    const bool coop = coop_min != NBUCKET;
     auto kern = coop ? (minb == 8   ? k_chem_batched<NS, 8, true>
                         : minb == 6 ? k_chem_batched<NS, 6, true>
                         : minb == 5 ? k_chem_batched<NS, 5, true>
@@ -401,26 +484,30 @@ static cudaError_t chem_batched_impl(double* U, int64_t cs, const int64_t* idx, 
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bs, 0);
     if (per_sm < 1) per_sm = 1;
-    int64_t blocks = (int64_t)sm_count * per_sm;
-    const int64_t need = (count + bs - 1) / bs;
-    if (blocks > need) blocks = need;
-    if (blocks < 1) blocks = 1;
+    const int64_t most = (int64_t)sm_count * per_sm;
+    int64_t blocks = std::min(most, std::max<int64_t>(1, (count + bs - 1) / bs));
+    // cells the cooperative queue may take: one per group of 8 lanes of the launch; under the
+    // automatic rule the launch has a group for every cell of a small batch
+    unsigned long long cap = (unsigned long long)blocks * (bs / 8);
+    if (coop_min == COOP_AUTO) {
+        blocks = std::min(most, std::max<int64_t>(1, (count + bs / 8 - 1) / (bs / 8)));
+        cap = (unsigned long long)blocks * (bs / 8);
+    }
     const unsigned long long* coop_n = nullptr;
     if (cost && order) {
-        cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * (NBUCKET + 1), s);
+        cudaError_t e = cudaMemsetAsync(bins, 0, sizeof(unsigned long long) * (NBIN + 2), s);
         if (e != cudaSuccess) return e;
         const int g = sm_count * 4;
-        const unsigned long long cap = (unsigned long long)blocks * (bs / 32) * 4;  // 4 groups per warp
         k_order_hist<<<g, 256, 0, s>>>(cost, count, bins);
-        k_order_scan<<<1, 1, 0, s>>>(bins, cap, coop_min);
+        k_order_scan<<<1, 1, 0, s>>>(bins, cap, coop_min == COOP_AUTO ? -1 : coop_min, 4 * sm_count);
         k_order_scatter<<<g, 256, 0, s>>>(cost, count, bins, order);
         *launches += 3;
-        coop_n = bins + NBUCKET;
+        coop_n = bins + NBIN;
     } else {
         order = nullptr;
     }
     kern<<<(unsigned)blocks, bs, 0, s>>>(U, cs, idx, order, count, dt, dt_dev, dtc, rtol, atol, trial, fail, h_hist,
-                                         cost, coop_n, st);
+                                         cost, coop_n, 128 * (int64_t)sm_count, st);
     ++*launches;
     return cudaGetLastError();
 }
@@ -448,12 +535,21 @@ cudaError_t launch_chem_batched(int ns, double* U, int64_t cs, const int64_t* id
                                            trial, fail, st, sm_count, s, launches);
 }
 
+// Batches of the plain and persistent forms up to this many cells per SM go to
+// k_chem_group: at 64 (9,728 cells) a group for each cell costs the FP64 pipe what the lanes'
+// step chains take (29,000 pipe cycles of a sub-partition an attempt against 450,000 for 32
+// lanes).  3,000 igniting cells: 6.6 ms in groups, 16.6 on lanes.
+constexpr int GROUP_CELLS_PER_SM = 64;
 template <int NS>
 static cudaError_t chem_impl(int form, double* U, int64_t cs, const int64_t* idx, int64_t count, double dt,
                              const double* dtc, double rtol, double atol, double* trial, int* fail, DevStatus* st,
                              int sm_count, cudaStream_t s, int64_t* launches, const double* dt_dev) {
     const int bs = 64;
-    if (form == HF_CHEM_PLAIN) {
+    if (count <= (int64_t)sm_count * GROUP_CELLS_PER_SM) {
+        // every cell in a group of 8 lanes; both forms, so that they stay bit-identical
+        const int64_t blocks = std::min<int64_t>((count + 7) / 8, (int64_t)sm_count * 4);
+        k_chem_group<NS><<<(unsigned)blocks, bs, 0, s>>>(U, cs, idx, count, dt, dt_dev, dtc, rtol, atol, trial, fail, st);
+    } else if (form == HF_CHEM_PLAIN) {
         k_chem_plain<NS><<<(unsigned)((count + bs - 1) / bs), bs, 0, s>>>(U, cs, idx, count, dt, dt_dev, dtc, rtol, atol,
                                                                           trial, fail, st);
     } else {
@@ -599,7 +695,7 @@ extern "C" hf_status hf_fastmath_eval(const double* x, int64_t n, double* exp_ou
     return cudaGetLastError() == cudaSuccess ? HF_OK : HF_ERR_CUDA;
 }
 extern "C" hf_status hf_set_chem_tuning(int32_t blocks_per_sm, int32_t coop_min_bucket) {
-    if (blocks_per_sm < 0 || coop_min_bucket < 0 || coop_min_bucket > 16 ||
+    if (blocks_per_sm < 0 || coop_min_bucket < 0 || coop_min_bucket > hf::COOP_AUTO ||
         (blocks_per_sm && blocks_per_sm != 4 && blocks_per_sm != 5 && blocks_per_sm != 6 && blocks_per_sm != 8))
         return HF_ERR_ARG;
     int m = 0, c = 0;
@@ -663,8 +759,10 @@ extern "C" hf_status hf_chem_advance_noalloc(int nspecies, double* U, int64_t co
         cudaMemsetAsync(&S->st.bad_cell, 0xff, sizeof(unsigned long long), s) != cudaSuccess)
         return HF_ERR_CUDA;
     int64_t launches = 0;
-    if (launch_chem(nspecies, HF_CHEM_PLAIN, U, comp_stride, cell_index, count, dt, dt_cell, rtol, atol, S->trial,
-                    S->fail, &S->st, 1, s, &launches) != cudaSuccess)
+    int sms = 1;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        launch_chem(nspecies, HF_CHEM_PLAIN, U, comp_stride, cell_index, count, dt, dt_cell, rtol, atol, S->trial,
+                    S->fail, &S->st, sms, s, &launches) != cudaSuccess)
         return HF_ERR_CUDA;
     DevStatus h;
     if (cudaMemcpyAsync(&h, &S->st, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||

@@ -190,12 +190,11 @@ __device__ __noinline__ bool solve_T_slow(const double* w, double et, double& T,
 // coefficients (a sum over species for each power of T) are most of what is left: 90 FP64
 // instructions a solve.  States near T_mid, outside [T_LO, T_HI], or whose FP32 phase does
 // not settle take solve_T_any.
-template <int NS, bool MASS>
-__device__ __forceinline__ bool solve_T_from(const double* w, double et, bool low, float t, double& T, double* m,
-                                             double& cv) {
+//
+// newton_T: the Newton steps from mixture coefficients m of the range `low` names; false
+// (T the FP32 phase's result, or as it came) when the state needs solve_T_any.
+__device__ __forceinline__ bool newton_T(const double* m, double et, bool low, float t, double& T, double& cv) {
     const float etf = fp_to_f32(et);
-    if (low) mix_coef_r<NS, 0, MASS>(w, m);
-    else mix_coef_r<NS, 1, MASS>(w, m);
     float mf[6], dt = 0.0f;
 #pragma unroll
     for (int j = 0; j < 6; ++j) mf[j] = fp_to_f32(m[j]);
@@ -238,8 +237,17 @@ __device__ __forceinline__ bool solve_T_from(const double* w, double et, bool lo
             return true;
         }
     }
+    if (fine) T = fp_from_f32(t);
+    return false;
+}
+template <int NS, bool MASS>
+__device__ __forceinline__ bool solve_T_from(const double* w, double et, bool low, float t, double& T, double* m,
+                                             double& cv) {
+    if (low) mix_coef_r<NS, 0, MASS>(w, m);
+    else mix_coef_r<NS, 1, MASS>(w, m);
+    if (newton_T(m, et, low, t, T, cv)) return true;
     // through copies, so that the arrays of the fast path stay in registers
-    double ws[NS], ms[6], Ts = fine ? fp_from_f32(t) : T, cvs = 0.0;
+    double ws[NS], ms[6], Ts = T, cvs = 0.0;
 #pragma unroll
     for (int k = 0; k < NS; ++k) ws[k] = w[k];
     const bool ok = solve_T_slow<NS, MASS>(ws, et, Ts, ms, cvs);

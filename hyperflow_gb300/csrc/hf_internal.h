@@ -14,6 +14,7 @@ struct DevStatus {
     unsigned long long rate_bits;  // CFL: max rate as the bits of a non-negative double
     unsigned long long counter;    // work-queue head / generic counter
     unsigned long long coop_counter;  // head of the batched chemistry's cooperative queue
+    unsigned long long costly_counter;  // head of its queue of costly cells
     unsigned long long steps;      // integrator steps (accepted + rejected)
     unsigned long long repairs;
     unsigned long long coop_cells;  // cells the batched chemistry took in groups of 8 lanes
@@ -166,7 +167,7 @@ cudaError_t launch_chem(int ns, int form, double* U, int64_t comp_stride, const 
 // dt_dev (nullable): read the interval from device memory instead of dt
 // bins: CHEM_BINS unsigned long long of device scratch (cost buckets and the size of the
 // cooperative queue)
-constexpr int CHEM_BINS = 32;
+constexpr int CHEM_BINS = 160;
 cudaError_t launch_chem_batched(int ns, double* U, int64_t cs, const int64_t* idx, int64_t count, double dt,
                                 const double* dt_dev, const double* dtc, double rtol, double atol, double* h_hist,
                                 int32_t* cost, int32_t* order, unsigned long long* bins, double* trial, int* fail,

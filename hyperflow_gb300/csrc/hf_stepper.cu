@@ -189,7 +189,7 @@ cudaError_t enqueue_step(hf_stepper* st, double cfl, double* S0, double* T1, dou
     HF_Q(phase_mark(st, rec, 1, s, nl));
     // react(dt): work-queue head reset, then the chemistry kernel of the stepper's form,
     // commit, validate
-    HF_Q(cudaMemsetAsync(&st->gst->counter, 0, 2 * sizeof(unsigned long long), s));  // work-queue heads
+    HF_Q(cudaMemsetAsync(&st->gst->counter, 0, 3 * sizeof(unsigned long long), s));  // work-queue heads
     if (st->chemistry) {
         if (st->chem_form == HF_CHEM_PLAIN) {  // the drop-in form: one thread per cell
             HF_Q(launch_chem(st->ns, HF_CHEM_PLAIN, X, P.comp_stride, st->cells, nc, 0.0, nullptr, st->rtol, st->atol,

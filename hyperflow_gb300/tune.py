@@ -3,7 +3,8 @@
 * Chemistry (hf_set_chem_tuning): the blocks of 64 lanes per SM the batched queue kernel
   is built for (its per-lane register budget) and the cooperative threshold (cells that
   took at least 2^b - 1 step attempts in the previous call are integrated by groups of 8
-  lanes, 4 cells per warp; 16, the default: never, and the kernel without that phase).
+  lanes, 4 cells per warp; 16: never, and the kernel without that phase; 17, what the library
+  starts with: its own choice of cells from their costs).
   Each candidate runs the batched chemistry three times on the same sample call (the
   chemistry input of a Strang step of the workload): the first two build the per-cell
   history (cost order, warm-started step sizes) as consecutive steps do, the third is
@@ -32,9 +33,9 @@ from . import _lib as L
 from . import solver as S
 
 CHEM_DEFAULT = (4, 16)
-CHEM_CANDIDATES = [CHEM_DEFAULT, (5, 16), (6, 16), (8, 16), (4, 3), (4, 5), (4, 7)]
+CHEM_CANDIDATES = [CHEM_DEFAULT, (4, 17), (5, 16), (6, 16), (8, 16), (4, 3), (4, 5), (4, 7)]
 MARGIN = 0.03
-STEP_CANDIDATES = [CHEM_DEFAULT, (4, 3), (4, 5), (4, 7)]
+STEP_CANDIDATES = [CHEM_DEFAULT, (4, 17), (4, 3), (4, 5), (4, 7)]
 
 
 def pick(sweep, key, default=CHEM_DEFAULT, margin=MARGIN):
