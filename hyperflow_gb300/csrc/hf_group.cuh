@@ -199,6 +199,7 @@ struct Cell {
     static constexpr int NI = NS - NQ;
     double y, yN2, Cin[NI];
     double h, t, tend, rho, ir, et, T;
+    double hu;  // step size of the last attempt
     double mom[3];
     int steps, attempts;
     bool active, rejectLast, rejectMore, fresh;
@@ -287,9 +288,11 @@ __device__ __forceinline__ double falloff(const Slot& s, const Kin& kc, double k
     return k;
 }
 
-// The lane's reactions into shared memory: q, and with JAC also T dq/dT and the partials.
+// The lane's reactions into shared memory: q, and with JAC also T dq/dT, the partials and
+// (where qo is given) the rates of progress with the slots' own rate constants.
 template <int rnd, bool JAC>
-__device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X, double M1, double M2, Shared* sh) {
+__device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X, double M1, double M2, Shared* sh,
+                                               double* qo) {
     const int t = lane8();
     {
         const int r = rnd * G + t;
@@ -308,6 +311,7 @@ __device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X
                 if constexpr (JAC) Tdk *= M;
             }
         }
+        const double own = k;
         if constexpr (round_has_dup(rnd)) {
             const double kn = __shfl_down_sync(FULL, k, 1, 8);
             if (s.dup == 1) k += kn;
@@ -342,6 +346,7 @@ __device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X
             double hh = (hc + hd) - (ha + hb);
             if constexpr (round_has_dn(rnd)) hh -= s.dn == 1 ? 1.0 : s.dn == -1 ? -1.0 : 0.0;
             sh->q[r] = k * net;
+            if (qo) qo[r] = own * net;
             sh->qT[r] = fma(kr * cc, hh, Tdk * net);
             double* v = sh->v + r * NVAL;
             v[0] = k * Cb;
@@ -354,12 +359,13 @@ __device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X
     }
 }
 template <bool JAC>
-__device__ __forceinline__ void reactions(const Kin& kc, double C, double M1, double M2, Shared* sh) {
+__device__ __forceinline__ void reactions(const Kin& kc, double C, double M1, double M2, Shared* sh,
+                                          double* qo = nullptr) {
     static_assert(NROUND == 3, "three rounds of reactions");
     const double X = C * kc.eg;
-    reaction_round<0, JAC>(kc, C, X, M1, M2, sh);
-    reaction_round<1, JAC>(kc, C, X, M1, M2, sh);
-    reaction_round<2, JAC>(kc, C, X, M1, M2, sh);
+    reaction_round<0, JAC>(kc, C, X, M1, M2, sh, qo);
+    reaction_round<1, JAC>(kc, C, X, M1, M2, sh, qo);
+    reaction_round<2, JAC>(kc, C, X, M1, M2, sh, qo);
 }
 
 struct RhsOut {
@@ -599,6 +605,7 @@ __device__ __forceinline__ int attempt(Cell<NS>& c, double rtol, double atol, Sh
             c.h = c.tend - c.t;
             last = true;
         }
+        c.hu = c.h;
         if (++c.attempts > 4 * MAX_STEPS) {
             go = false;
             res = CELL_MAXSTEPS;

@@ -1,9 +1,8 @@
-// Per-cell chemistry device code shared by the forward chemistry kernels
-// (hf_chem.cu) and the discrete adjoint (hf_adjoint.cu): NASA7 species thermo,
-// mass-action kinetics of the generated H2_Li table with its analytic Jacobian,
-// the constant-(rho, e) right-hand side of HyperFlow_V3/src/chemistry.cpp:36-53,
-// and the Rodas4 cell integrator (Hairer & Wanner, Solving ODEs II, Sec. VI.7,
-// KPP coefficient ordering and step controller).
+// Device code shared by the chemistry kernels (hf_chem.cu) and the discrete adjoint
+// (hf_adjoint.cu): NASA7 species thermo, mass-action rates of the generated H2_Li table as
+// the tagging kernel and the objectives' derivatives use them, and the Rodas4 tableau
+// (Hairer & Wanner, Solving ODEs II, Sec. VI.7, KPP coefficient ordering).  The integrators
+// are in hf_cell.cuh (one cell per lane) and hf_group.cuh (one per group of 8 lanes).
 //
 // Pre-exponential factors live in __constant__ memory, one copy per translation
 // unit (static); each unit that includes this header uploads them with
@@ -272,120 +271,6 @@ __device__ __forceinline__ void all_rates(const KinCtx<NS>& kc, const double* C,
     (add_rate<(int)Rs, NS>(kc, C, w), ...);
 }
 
-// d(w_i)/dC_m into JC[i][m] (rows i < NS-1), d(w_i)/dT into JT[i]; with W, also the
-// rate of progress into w exactly as add_rate computes it (same k, 1/Kc, products).
-template <int R, int NS, bool W = false>
-__device__ __forceinline__ void add_jac(const KinCtx<NS>& kc, const double* C, double* JC, double* JT,
-                                        double* w = nullptr) {
-    constexpr Reaction rx = RXN[R];
-    constexpr int N = NS - 1;
-    const double kinf = c_A[R] * kinf_T<R, NS>(kc);
-    const double dlnkinf = rx.b * kc.invT + rx.EaR * kc.invT * kc.invT;
-    double k, dkdT, dkdM = 0.0, M = 0.0;
-    if constexpr (rx.type == RXN_ELEMENTARY) {
-        k = kinf;
-        dkdT = kinf * dlnkinf;
-    } else if constexpr (rx.type == RXN_THREE_BODY) {
-        M = third_body<R, NS>(C, kc.Csum);
-        k = kinf * M;
-        dkdT = k * dlnkinf;
-        dkdM = kinf;
-    } else {
-        M = third_body<R, NS>(C, kc.Csum);
-        const double k0 = c_A0[R] * k0_T<R, NS>(kc);
-        const double dlnk0 = rx.b0 * kc.invT + rx.Ea0R * kc.invT * kc.invT;
-        const double Pr = k0 * M / kinf;
-        double dPr, dTF;
-        const double lF = troe_log10F<R>(kc.T, Pr, &dPr, &dTF);
-        const double F = fexp(lF * fm::LN10);
-        const double dlnk_dlnPr = 1.0 - Pr / (1.0 + Pr) + dPr;
-        k = kinf * (Pr / (1.0 + Pr)) * F;
-        dkdT = k * (dlnkinf + dlnk_dlnPr * (dlnk0 - dlnkinf) + dTF);
-        dkdM = M > 0.0 ? k * dlnk_dlnPr / M : k0 * F;
-    }
-    const double ikc = inv_kc<R, NS>(kc);
-    if constexpr (W) {
-        double pf = k, pr = k * ikc;
-#pragma unroll
-        for (int i = 0; i < rx.nreac; ++i) pf *= C[rx.reac[i]];
-#pragma unroll
-        for (int i = 0; i < rx.nprod; ++i) pr *= C[rx.prod[i]];
-        const double q = pf - pr;
-#pragma unroll
-        for (int i = 0; i < rx.nreac; ++i) w[rx.reac[i]] -= q;
-#pragma unroll
-        for (int i = 0; i < rx.nprod; ++i) w[rx.prod[i]] += q;
-    }
-    double Pf = 1.0, Pb = 1.0;
-#pragma unroll
-    for (int i = 0; i < rx.nreac; ++i) Pf *= C[rx.reac[i]];
-#pragma unroll
-    for (int i = 0; i < rx.nprod; ++i) Pb *= C[rx.prod[i]];
-    const double net = Pf - ikc * Pb;
-    // dlnKc/dT = sum nu h/RT / T - dn / T  (d(g/RT)/dT = -h/(R T^2))
-    double dh = 0.0;
-#pragma unroll
-    for (int i = 0; i < rx.nprod; ++i) dh += kc.hRT[rx.prod[i]];
-#pragma unroll
-    for (int i = 0; i < rx.nreac; ++i) dh -= kc.hRT[rx.reac[i]];
-    constexpr int dn = rx.nprod - rx.nreac;
-    const double dlnKc = (dh - (double)dn) * kc.invT;
-    const double dqdT = dkdT * net + k * ikc * dlnKc * Pb;
-    // dq/dC_m (mass action part) for participants
-    double dq[NS];
-#pragma unroll
-    for (int m = 0; m < NS; ++m) dq[m] = 0.0;
-#pragma unroll
-    for (int i = 0; i < rx.nreac; ++i) {
-        double p = k;
-#pragma unroll
-        for (int j = 0; j < rx.nreac; ++j)
-            if (j != i) p *= C[rx.reac[j]];
-        dq[rx.reac[i]] += p;
-    }
-#pragma unroll
-    for (int i = 0; i < rx.nprod; ++i) {
-        double p = k * ikc;
-#pragma unroll
-        for (int j = 0; j < rx.nprod; ++j)
-            if (j != i) p *= C[rx.prod[j]];
-        dq[rx.prod[i]] -= p;
-    }
-    if constexpr (rx.type != RXN_ELEMENTARY) {
-        const double t = dkdM * net;
-#pragma unroll
-        for (int m = 0; m < NS; ++m) dq[m] = fma(t, rx.eff[m], dq[m]);
-    }
-#pragma unroll
-    for (int i = 0; i < rx.nreac; ++i) {
-        const int s = rx.reac[i];
-        if (s < N) {
-            JT[s] -= dqdT;
-#pragma unroll
-            for (int m = 0; m < NS; ++m) JC[s * NS + m] -= dq[m];
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < rx.nprod; ++i) {
-        const int s = rx.prod[i];
-        if (s < N) {
-            JT[s] += dqdT;
-#pragma unroll
-            for (int m = 0; m < NS; ++m) JC[s * NS + m] += dq[m];
-        }
-    }
-}
-template <int NS, size_t... Rs>
-__device__ __forceinline__ void all_jac(const KinCtx<NS>& kc, const double* C, double* JC, double* JT,
-                                        std::index_sequence<Rs...>) {
-    (add_jac<(int)Rs, NS>(kc, C, JC, JT), ...);
-}
-template <int NS, size_t... Rs>
-__device__ __forceinline__ void all_jac_rates(const KinCtx<NS>& kc, const double* C, double* JC, double* JT,
-                                              double* w, std::index_sequence<Rs...>) {
-    (add_jac<(int)Rs, NS, true>(kc, C, JC, JT, w), ...);
-}
-
 // ---------------------------------------------------------------- ODE pieces
 // composition of y (Y_0..Y_{N-1}; last species closes) -> z = Y/W, C = rho Y/W
 template <int NS>
@@ -399,63 +284,6 @@ __device__ __forceinline__ void comp(const double* y, double rho, double* z, dou
     }
     z[NS - 1] = (1.0 - s) * INVW.v[NS - 1];
     C[NS - 1] = rho * z[NS - 1];
-}
-
-// chemistry.cpp:36-53
-template <int NS>
-__device__ __noinline__ bool chem_rhs(double rho, double e, double& T, const double* y, double* dy) {
-    double z[NS], C[NS], m[6];
-    comp<NS>(y, rho, z, C);
-    double Tn = T;
-    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
-    T = Tn;
-    KinCtx<NS> kc;
-    kin_setup<NS>(T, C, kc);
-    double w[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) w[k] = 0.0;
-    all_rates<NS>(kc, C, w, std::make_index_sequence<NR>{});
-    bool ok = true;
-    const double ir = 1.0 / rho;
-#pragma unroll
-    for (int k = 0; k < NS - 1; ++k) {
-        dy[k] = w[k] * D_MW.v[k] * ir;
-        ok = ok && isfinite(dy[k]);
-    }
-    return ok;
-}
-
-template <int NS>
-__device__ __noinline__ bool chem_jac(double rho, double e, double& T, const double* y, double* J) {
-    constexpr int N = NS - 1, L = NS - 1;
-    double z[NS], C[NS], m[6];
-    comp<NS>(y, rho, z, C);
-    double Tn = T;
-    if (!solve_T_iter<NS>(z, e, Tn, m)) return false;
-    T = Tn;
-    KinCtx<NS> kc;
-    kin_setup<NS>(T, C, kc);
-    double JC[N * NS], JT[N];
-#pragma unroll
-    for (int i = 0; i < N * NS; ++i) JC[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) JT[i] = 0.0;
-    all_jac<NS>(kc, C, JC, JT, std::make_index_sequence<NR>{});
-    // dT/dy_j = -(e_j - e_L)/cv, e_k = R T/W_k (h_k/RT - 1)
-    const double cv = poly_cv(m, T);  // cv/R in the z-weighted units of the mixture
-    double dTdy[N];
-    const double eL = (kc.hRT[L] - 1.0) * INVW.v[L];
-#pragma unroll
-    for (int j = 0; j < N; ++j) dTdy[j] = -T * ((kc.hRT[j] - 1.0) * INVW.v[j] - eL) / cv;
-    const double ir = 1.0 / rho;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const double cl = JC[i * NS + L] * INVW.v[L];
-        const double ti = JT[i] * ir;
-#pragma unroll
-        for (int j = 0; j < N; ++j) J[i * N + j] = D_MW.v[i] * (JC[i * NS + j] * INVW.v[j] - cl + ti * dTdy[j]);
-    }
-    return true;
 }
 
 // ---------------------------------------------------------------- Rodas4
@@ -474,49 +302,5 @@ constexpr double RGAMMA = 0.25;
 constexpr long MAX_STEPS = 5000;
 
 enum : int { CELL_CONTINUE = 0, CELL_DONE = 1, CELL_FAIL = 2, CELL_MAXSTEPS = 3 };
-
-// LU with partial pivoting in place (P A = L U); the diagonal holds 1/U_kk.
-template <int N>
-__device__ __forceinline__ bool lu_factor(double* A, int* piv) {
-#pragma unroll 1
-    for (int k = 0; k < N; ++k) {
-        int p = k;
-        double best = fabs(A[k * N + k]);
-        for (int i = k + 1; i < N; ++i) {
-            const double v = fabs(A[i * N + k]);
-            if (v > best) { best = v; p = i; }
-        }
-        if (!(best > 0.0) || !isfinite(best)) return false;
-        piv[k] = p;
-        if (p != k) {
-#pragma unroll
-            for (int j = 0; j < N; ++j) { const double t = A[k * N + j]; A[k * N + j] = A[p * N + j]; A[p * N + j] = t; }
-        }
-        const double inv = 1.0 / A[k * N + k];
-        A[k * N + k] = inv;  // the solves multiply by the reciprocal pivot
-        for (int i = k + 1; i < N; ++i) {
-            const double l = A[i * N + k] * inv;
-            A[i * N + k] = l;
-            for (int j = k + 1; j < N; ++j) A[i * N + j] = fma(-l, A[k * N + j], A[i * N + j]);
-        }
-    }
-    return true;
-}
-template <int N>
-__device__ __forceinline__ void lu_solve(const double* A, const int* piv, double* b) {
-#pragma unroll 1
-    for (int k = 0; k < N; ++k) {
-        const int p = piv[k];
-        if (p != k) { const double t = b[k]; b[k] = b[p]; b[p] = t; }
-    }
-#pragma unroll 1
-    for (int i = 1; i < N; ++i)
-        for (int j = 0; j < i; ++j) b[i] = fma(-A[i * N + j], b[j], b[i]);
-#pragma unroll 1
-    for (int i = N - 1; i >= 0; --i) {
-        for (int j = i + 1; j < N; ++j) b[i] = fma(-A[i * N + j], b[j], b[i]);
-        b[i] *= A[i * N + i];  // reciprocal pivot
-    }
-}
 
 }  // namespace hf
