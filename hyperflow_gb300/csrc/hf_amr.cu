@@ -9,6 +9,7 @@
 // fallback past REPAIR_CAP negative entries).
 #include <cstddef>
 #include <cstring>
+#include "hf_fp64.cuh"
 #include "hf_internal.h"
 
 namespace hf {
@@ -35,8 +36,10 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
 constexpr int TOT_BLOCK = 256;
 constexpr int TOT_GRID = 304;  // fixed partition: results independent of the device
 
-// Pass 1: block b sums the cells of a fixed contiguous range (all patches' cells in
-// order) into partial[b][n] (double-double, tree order fixed).
+// Pass 1: block (b, n) sums component n of the cells of a fixed contiguous range (all
+// patches' cells in order) into partial[b][n] (double-double, tree order fixed).  One block
+// to a component: a block's double-double tree is a chain of FP64 additions (64 cycles
+// each), which one block after another took 78 us for 12 components.
 __global__ void __launch_bounds__(TOT_BLOCK) k_totals(const hf_patch* __restrict__ patches, int npatch,
                                                       const double* __restrict__ U,
                                                       const uint8_t* __restrict__ mask, int64_t total, int nv,
@@ -44,7 +47,8 @@ __global__ void __launch_bounds__(TOT_BLOCK) k_totals(const hf_patch* __restrict
     __shared__ DD sh[TOT_BLOCK];
     const int64_t per_block = (total + gridDim.x - 1) / gridDim.x;
     const int64_t c0 = (int64_t)blockIdx.x * per_block, c1 = min(total, c0 + per_block);
-    for (int n = 0; n < nv; ++n) {
+    {
+        const int n = blockIdx.y;
         DD acc{0.0, 0.0};
         int p = 0;
         int64_t base = 0;
@@ -67,24 +71,29 @@ __global__ void __launch_bounds__(TOT_BLOCK) k_totals(const hf_patch* __restrict
             __syncthreads();
         }
         if (threadIdx.x == 0) partial[(int64_t)blockIdx.x * nv + n] = sh[0];
-        __syncthreads();
     }
 }
-// Pass 2: one thread per component adds the block partials in block order.
+// Pass 2: warp n adds the partials of component n (each lane a fixed stride of blocks, then
+// a fixed tree): a chain of 15 double-double additions where one thread took 304 (152 us).
 __global__ void k_totals_final(const DD* __restrict__ partial, int nblocks, int nv, double* __restrict__ out) {
-    const int n = threadIdx.x;
-    if (n >= nv) return;
+    const int n = blockIdx.x, lane = threadIdx.x;
     DD acc{0.0, 0.0};
-    for (int b = 0; b < nblocks; ++b) acc = dd_add(acc, partial[(int64_t)b * nv + n]);
-    out[n] = acc.hi + acc.lo;
+    for (int b = lane; b < nblocks; b += 32) acc = dd_add(acc, partial[(int64_t)b * nv + n]);
+    for (int o = 16; o > 0; o >>= 1) {
+        DD other;
+        other.hi = __shfl_down_sync(0xffffffffu, acc.hi, o);
+        other.lo = __shfl_down_sync(0xffffffffu, acc.lo, o);
+        acc = dd_add(acc, other);
+    }
+    if (lane == 0) out[n] = acc.hi + acc.lo;
 }
 
 cudaError_t launch_totals(const hf_patch* patches_dev, int npatch, int64_t total, const double* U, const uint8_t* mask,
                           int nv, double vol, int absolute, void* scratch, double* out_dev, cudaStream_t s,
                           int64_t* launches) {
     DD* partial = static_cast<DD*>(scratch);
-    k_totals<<<TOT_GRID, TOT_BLOCK, 0, s>>>(patches_dev, npatch, U, mask, total, nv, vol, absolute, partial);
-    k_totals_final<<<1, 32, 0, s>>>(partial, TOT_GRID, nv, out_dev);
+    k_totals<<<dim3(TOT_GRID, nv), TOT_BLOCK, 0, s>>>(patches_dev, npatch, U, mask, total, nv, vol, absolute, partial);
+    k_totals_final<<<nv, 32, 0, s>>>(partial, TOT_GRID, nv, out_dev);
     *launches += 2;
     return cudaGetLastError();
 }
@@ -230,6 +239,10 @@ cudaError_t launch_reflux(const Level& L, const hf_patch* coarse_dev, const hf_p
 // reference's order: levels in turn, the patches of a level in table order, the cells
 // of a patch row by row.  A cell is identified by its level and its patch-packed index
 // (base[p] + row-major index in patch p).
+//   find:        whether any leaf value is negative or not a number; the others return at
+//                once where none is (the usual stage: the scan's atomics, two per species
+//                and cell, took 90 us a launch, 8.7 of the 31 ms of four steps on three
+//                levels of 75,000 leaf cells)
 //   scan pass 0: per species the peak partial density and the largest mass
 //                (value x cell volume) over all leaf cells;
 //   scan pass 1: donor = the first cell (lowest level, then lowest index) holding that
@@ -247,7 +260,26 @@ __device__ __forceinline__ unsigned long long repair_key(int l, int64_t c) {
 }
 
 template <int NS>
+__global__ void k_crep_find(RepairLevel R, RepairScratch* rs) {
+    const hf_patch P = R.patches[blockIdx.y];
+    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (int64_t)P.nx * P.ny) return;
+    const int64_t c = R.base[blockIdx.y] + idx;
+    if (R.leaf && !R.leaf[c]) return;
+    const int i = (int)(idx % P.nx), j = (int)(idx / P.nx);
+    const int64_t g = P.offset + (int64_t)(j + P.ng) * P.pitch + (i + P.ng);
+    bool found = false;
+#pragma unroll
+    for (int n = 0; n < NS; ++n) {
+        const double v = R.U[g + n * P.comp_stride];
+        found = found || fp_neg(v) || fp_nan(v);
+    }
+    if (found) rs->found = 1;
+}
+
+template <int NS>
 __global__ void k_crep_scan(RepairLevel R, int l, int pass, RepairScratch* rs) {
+    if (!rs->found) return;
     const hf_patch P = R.patches[blockIdx.y];
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)P.nx * P.ny) return;
@@ -271,6 +303,7 @@ __global__ void k_crep_scan(RepairLevel R, int l, int pass, RepairScratch* rs) {
 
 template <int NS>
 __global__ void k_crep_apply(RepairLevel R, int l, RepairScratch* rs, DevStatus* st) {
+    if (!rs->found) return;
     const hf_patch P = R.patches[blockIdx.y];
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)P.nx * P.ny) return;
@@ -376,12 +409,15 @@ cudaError_t launch_composite_repair(int ns, const RepairLevels& R, RepairScratch
     cudaError_t e = cudaMemsetAsync(rs, 0, offsetof(RepairScratch, key), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(rs->donor, 0xff, sizeof(rs->donor), s);
     if (e != cudaSuccess) return e;
-    for (int pass = 0; pass < 3; ++pass)
+    for (int pass = -1; pass < 3; ++pass)
         for (int l = 0; l < R.nlev; ++l) {
             const RepairLevel& L = R.lev[l];
             if (L.npatch <= 0) continue;
             const dim3 grid((unsigned)((L.max_cells + 127) / 128), (unsigned)L.npatch);
-            if (pass < 2) {
+            if (pass < 0) {
+                if (ns == 9) k_crep_find<9><<<grid, 128, 0, s>>>(L, rs);
+                else k_crep_find<10><<<grid, 128, 0, s>>>(L, rs);
+            } else if (pass < 2) {
                 if (ns == 9) k_crep_scan<9><<<grid, 128, 0, s>>>(L, l, pass, rs);
                 else k_crep_scan<10><<<grid, 128, 0, s>>>(L, l, pass, rs);
             } else {

@@ -413,47 +413,65 @@ constexpr float GROUP_RATE = 33.8f, LANE_RATE = 97.0f, GROUP_ALONE = 73.0f, GROU
 __device__ __forceinline__ float bin_cost(int b) {  // attempts at the bin's lower edge
     return (float)(1u << (b / SUB)) * (1.0f + (float)(b % SUB) / SUB) - 1.0f;
 }
-__global__ void k_order_scan(unsigned long long* bins, unsigned long long cap, int min_bucket, int subparts) {
+// One block of NBIN threads: the bins and their costs in shared memory, suffix sums by
+// doubling, the line by one thread per candidate bin (45 us in one thread over global memory).
+__global__ void __launch_bounds__(NBIN) k_order_scan(unsigned long long* bins, unsigned long long cap, int min_bucket,
+                                                     int subparts) {
+    __shared__ unsigned long long cum[NBIN];  // cells of bins >= b
+    __shared__ float work[NBIN];              // their attempts
+    __shared__ float best_t[NBIN];
+    __shared__ int top, line;
+    const int b = threadIdx.x;
+    const unsigned long long n = bins[b];
+    cum[b] = n;
+    work[b] = (float)n * bin_cost(b);
+    if (b == 0) {
+        top = 0;
+        line = NBIN;
+    }
+    __syncthreads();
+    if (n) atomicMax(&top, b + 1);
+    for (int o = 1; o < NBIN; o <<= 1) {
+        const unsigned long long c = b + o < NBIN ? cum[b + o] : 0;
+        const float w = b + o < NBIN ? work[b + o] : 0.0f;
+        __syncthreads();
+        cum[b] += c;
+        work[b] += w;
+        __syncthreads();
+    }
     int min_bin = min_bucket * SUB;
     if (min_bucket < 0) {
-        float total = 0.0f, most = 0.0f;
-        unsigned long long costly = 0;
-        for (int b = 0; b < NBIN; ++b) {
-            total += (float)bins[b] * bin_cost(b);
-            if (bins[b]) most = bin_cost(b + 1);
-            if (b >= COSTLY_BUCKET * SUB) costly += bins[b];
+        const float r = 608.0f / (float)subparts, total = work[0], most = bin_cost(top);
+        const float p0 = total / LANE_RATE * r;
+        const float l0 = most * (cum[COSTLY_BUCKET * SUB] <= 32ull * subparts ? LANE_ALONE : LANE_PAIR);
+        const float p = (work[b] / GROUP_RATE + (total - work[b]) / LANE_RATE) * r;
+        const float g = most * (cum[b] <= 4ull * subparts ? GROUP_ALONE : GROUP_PAIR), l = bin_cost(b) * LANE_PAIR;
+        const float t = p * p + g * g + l * l;
+        best_t[b] = b >= SUB && n && cum[b] <= cap && t < p0 * p0 + l0 * l0 ? t : 3e38f;
+        __syncthreads();
+        for (int o = NBIN / 2; o > 0; o >>= 1) {
+            if (b < o) best_t[b] = fminf(best_t[b], best_t[b + o]);
+            __syncthreads();
         }
-        const float r = 608.0f / (float)subparts;
-        min_bin = NBIN;
-        const float p0 = total / LANE_RATE * r, l0 = most * (costly <= 32ull * subparts ? LANE_ALONE : LANE_PAIR);
-        float best = p0 * p0 + l0 * l0;
-        float grp = 0.0f;
-        unsigned long long n = 0;
-        for (int b = NBIN - 1; b >= 3 * SUB; --b) {
-            n += bins[b];
-            if (n > cap) break;
-            grp += (float)bins[b] * bin_cost(b);
-            const float p = (grp / GROUP_RATE + (total - grp) / LANE_RATE) * r;
-            const float g = most * (n <= 4ull * subparts ? GROUP_ALONE : GROUP_PAIR), l = bin_cost(b) * LANE_PAIR;
-            const float t = p * p + g * g + l * l;
-            if (bins[b] && t < best) {
-                best = t;
-                min_bin = b;
-            }
-        }
+        if (best_t[0] < 3e38f && b >= SUB && n && cum[b] <= cap && t == best_t[0]) atomicMin(&line, b);
+        __syncthreads();
+        min_bin = line;
     }
-    unsigned long long off = 0, ncoop = 0, costly = 0;
-    bool open = true;
-    for (int b = NBIN - 1; b >= 0; --b) {
-        const unsigned long long n = bins[b];
-        if (open && b >= min_bin && ncoop + n <= cap) ncoop += n;
-        else open = false;
-        if (!open && b >= COSTLY_BUCKET * SUB) costly += n;
-        bins[b] = off;
-        off += n;
+    // whole bins from the top down to min_bin while they fit
+    const bool coop = b >= min_bin && cum[b] <= cap;
+    __syncthreads();
+    const unsigned long long above = b + 1 < NBIN ? cum[b + 1] : 0;
+    bins[b] = above;
+    __shared__ unsigned long long ncoop;
+    if (b == 0) ncoop = 0;
+    __syncthreads();
+    if (coop) atomicMax(&ncoop, cum[b]);
+    __syncthreads();
+    if (b == 0) {
+        bins[NBIN] = ncoop;
+        const unsigned long long hi = cum[COSTLY_BUCKET * SUB];
+        bins[NBIN + 1] = hi > ncoop ? hi - ncoop : 0;
     }
-    bins[NBIN] = ncoop;
-    bins[NBIN + 1] = costly;
 }
 __global__ void k_order_scatter(const int32_t* __restrict__ cost, int64_t count, unsigned long long* __restrict__ bins,
                                 int32_t* __restrict__ order) {
@@ -499,7 +517,7 @@ static cudaError_t chem_batched_impl(double* U, int64_t cs, const int64_t* idx, 
         if (e != cudaSuccess) return e;
         const int g = sm_count * 4;
         k_order_hist<<<g, 256, 0, s>>>(cost, count, bins);
-        k_order_scan<<<1, 1, 0, s>>>(bins, cap, coop_min == COOP_AUTO ? -1 : coop_min, 4 * sm_count);
+        k_order_scan<<<1, NBIN, 0, s>>>(bins, cap, coop_min == COOP_AUTO ? -1 : coop_min, 4 * sm_count);
         k_order_scatter<<<g, 256, 0, s>>>(cost, count, bins, order);
         *launches += 3;
         coop_n = bins + NBIN;

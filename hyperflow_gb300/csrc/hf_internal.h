@@ -218,6 +218,7 @@ struct RepairScratch {  // device memory, cleared by every launch_composite_repa
     unsigned long long mass_bits[16];
     double deficit[16];          // atomic deficit sums (used past REPAIR_CAP entries)
     unsigned long long count;    // negative entries found
+    unsigned long long found;    // 1: some leaf value is negative or not a number
     unsigned long long donor[16];
     unsigned long long key[REPAIR_CAP];  // species << 60 | level << 52 | cell
     double val[REPAIR_CAP];              // deficit of the entry (-value x volume)
