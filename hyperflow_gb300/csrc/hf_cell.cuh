@@ -20,8 +20,11 @@
 //    leaves the registers; every attempt starts with it.  A rejected step evaluates J
 //    again, which costs nothing: the lanes of its warp that accepted theirs, or hold a new
 //    cell, need it anyway.
-// About 5,700 FP64 instructions an attempt against 13,900 with mass-fraction unknowns, J
-// kept beside its factors, 11-instruction exponentials and two FP64 Newton steps.
+//  * Species' g relative to the elements as H2 and O2, and the inert species' share of the
+//    mixture polynomial kept with the cell.
+// About 5,100 FP64 instructions an attempt against 13,900 with mass-fraction unknowns, J
+// kept beside its factors, 11-instruction exponentials and two FP64 Newton steps; 206 us an
+// attempt with the sub-partition to itself, 377 beside a second warp (then the pipe is full).
 #pragma once
 #include "hf_exptab.h"
 #include "hf_kinetics.cuh"
@@ -163,7 +166,7 @@ constexpr NetNu make_nu() {
 }
 __device__ constexpr NetNu D_NU = make_nu();
 // g_k = a0 (1 - lnT) + a5/T - a6 + c1 T + c2 T^2 + c3 T^3 + c4 T^4
-struct GCoef { double c[2][NQ][5]; };
+struct GCoef { double c[2][NQ][7]; };  // -a6, c1..c4, a0, a5
 constexpr GCoef make_gcoef() {
     GCoef g{};
     for (int r = 0; r < 2; ++r)
@@ -174,27 +177,52 @@ constexpr GCoef make_gcoef() {
             g.c[r][k][2] = -a[2] / 6.0;
             g.c[r][k][3] = -a[3] / 12.0;
             g.c[r][k][4] = -a[4] / 20.0;
+            g.c[r][k][5] = a[0];
+            g.c[r][k][6] = a[5];
         }
     return g;
 }
 __device__ constexpr GCoef D_GCOEF = make_gcoef();
+// The same relative to the elements as H2 and O2: g_k - n_H/2 g_H2 - n_O/2 g_O2.  Reactions
+// conserve both elements, so equilibrium constants are unchanged, and H2 and O2 need no
+// exponential (six pairs instead of eight).
+constexpr int ATOMS_H[NQ] = {2, 0, 2, 1, 0, 1, 1, 2}, ATOMS_O[NQ] = {0, 2, 1, 0, 1, 1, 2, 2};
+constexpr int NREF = 2;  // species 0 and 1
+constexpr bool conserves() {
+    for (int r = 0; r < NR; ++r) {
+        int h = 0, o = 0;
+        for (int i = 0; i < RXN[r].nreac; ++i) { h -= ATOMS_H[RXN[r].reac[i]]; o -= ATOMS_O[RXN[r].reac[i]]; }
+        for (int i = 0; i < RXN[r].nprod; ++i) { h += ATOMS_H[RXN[r].prod[i]]; o += ATOMS_O[RXN[r].prod[i]]; }
+        if (h != 0 || o != 0) return false;
+    }
+    return true;
+}
+static_assert(conserves(), "species 0 and 1 as element references");
+constexpr GCoef make_gref() {
+    const GCoef g = make_gcoef();
+    GCoef d{};
+    for (int r = 0; r < 2; ++r)
+        for (int k = 0; k < NQ; ++k)
+            for (int j = 0; j < 7; ++j)
+                d.c[r][k][j] = g.c[r][k][j] - 0.5 * ATOMS_H[k] * g.c[r][0][j] - 0.5 * ATOMS_O[k] * g.c[r][1][j];
+    return d;
+}
+__device__ constexpr GCoef D_GREF = make_gref();
 
 // T-dependent quantities of one evaluation.
 struct Kin {
     double T, invT, lnT, rt, irt;  // rt = R T / p0, irt = 1 / rt
-    double eg[NQ], ieg[NQ];        // exp(g_k), exp(-g_k)
+    double eg[NQ], ieg[NQ];        // exp(g_k), exp(-g_k), g relative to H2 and O2 (theirs: 1, unused)
     double ar[NEXP];
 };
 template <int RG>
 __device__ __forceinline__ void g_of_T(double T, double lnT, double invT, double* g) {
     const double om = 1.0 - lnT;
 #pragma unroll
-    for (int k = 0; k < NQ; ++k) {
-        const double* a = D_NASA.c[RG][k];
-        const double* c = D_GCOEF.c[RG][k];
-        double p = c[0];
-        if (c[1] != 0.0 || c[4] != 0.0) p = fma(T, fma(T, fma(T, fma(T, c[4], c[3]), c[2]), c[1]), c[0]);
-        g[k] = fma(a[0], om, fma(a[5], invT, p));
+    for (int k = NREF; k < NQ; ++k) {
+        const double* c = D_GREF.c[RG][k];
+        const double p = fma(T, fma(T, fma(T, fma(T, c[4], c[3]), c[2]), c[1]), c[0]);
+        g[k] = fma(c[5], om, fma(c[6], invT, p));
     }
 }
 template <int RG>
@@ -219,7 +247,7 @@ __device__ __forceinline__ void kin_at(double T, Kin& k) {
     else g_of_T<1>(T, k.lnT, k.invT, g);
     // rolled: one body of each exponential, for the instruction cache
 #pragma unroll 1
-    for (int s = 0; s < NQ; ++s) fexp_pair(g[s], k.eg[s], k.ieg[s]);
+    for (int s = NREF; s < NQ; ++s) fexp_pair(g[s], k.eg[s], k.ieg[s]);
 #pragma unroll 1
     for (int i = 0; i < NEXP; ++i) {
         double x = -D_SLOTS.E[i] * k.invT;
@@ -288,6 +316,37 @@ __device__ __forceinline__ double falloff(const Kin& kc, double M, double& Tdk, 
     return k;
 }
 
+// prod_reac exp(-g) (RT/p0)^dn: the factor of prod_prod X in the reverse rate.
+template <int R>
+__device__ __forceinline__ double ieg_factor(const Kin& kc) {
+    constexpr Reaction rx = RXN[R];
+    constexpr int dn = rx.nprod - rx.nreac;
+    double b = 1.0;
+    bool set = false;
+    auto mul = [&](double v) {
+        b = set ? b * v : v;
+        set = true;
+    };
+    if constexpr (rx.reac[0] >= NREF) mul(kc.ieg[rx.reac[0]]);
+    if constexpr (rx.nreac == 2) {
+        if constexpr (rx.reac[1] >= NREF) mul(kc.ieg[rx.reac[1]]);
+    }
+    if constexpr (dn == 1) mul(kc.rt);
+    if constexpr (dn == -1) mul(kc.irt);
+    return b;
+}
+// ... and with prod_prod exp(g): 1 / Kc
+template <int R>
+__device__ __forceinline__ double inv_kc_factor(const Kin& kc) {
+    constexpr Reaction rx = RXN[R];
+    double b = ieg_factor<R>(kc);
+    if constexpr (rx.prod[0] >= NREF) b *= kc.eg[rx.prod[0]];
+    if constexpr (rx.nprod == 2) {
+        if constexpr (rx.prod[1] >= NREF) b *= kc.eg[rx.prod[1]];
+    }
+    return b;
+}
+
 // ---------------------------------------------------------------- right-hand side
 template <int R, int NS>
 __device__ __forceinline__ void rate(const Kin& kc, const double* C, const double* X, double Csum, double* w) {
@@ -303,15 +362,11 @@ __device__ __forceinline__ void rate(const Kin& kc, const double* C, const doubl
             if constexpr (rx.type == RXN_THREE_BODY) k *= third<R, NS>(C, Csum);
         }
         constexpr int dn = rx.nprod - rx.nreac;
-        double b = kc.ieg[rx.reac[0]], f = C[rx.reac[0]];
-        if constexpr (rx.nreac == 2) {
-            b *= kc.ieg[rx.reac[1]];
-            f *= C[rx.reac[1]];
-        }
-        if constexpr (dn == 1) b *= kc.rt;
-        if constexpr (dn == -1) b *= kc.irt;
+        double f = C[rx.reac[0]];
+        if constexpr (rx.nreac == 2) f *= C[rx.reac[1]];
+        double b = X[rx.prod[0]];
         if constexpr (rx.nprod == 2) b *= X[rx.prod[1]];
-        const double q = k * fma(-b, X[rx.prod[0]], f);
+        const double q = k * fma(-ieg_factor<R>(kc), b, f);
 #pragma unroll
         for (int s = 0; s < NQ; ++s) {
             if (D_NU.v[R][s] == 1) w[s] += q;
@@ -332,6 +387,7 @@ struct Cell {
     static constexpr int N = NS - 1, NI = NS - NQ;
     double y[N];     // mass fractions (the last species closes)
     double Cin[NI];  // concentrations of the inert species (constant over the interval)
+    double mi[2][6], Ci;  // their mixture coefficients in both NASA ranges, and total
     double h, t, tend, rho, ir, e, et, T;  // et = rho e / R; T: of y, or near it
     double mom[3];   // rho*u, rho*v, rho*E: chemistry leaves them unchanged
     int steps, attempts;
@@ -340,16 +396,26 @@ struct Cell {
 
 template <int NS>
 __device__ __forceinline__ bool weights_T(const Cell<NS>& c, const double* C, double& T, double& cv, double& Csum) {
-    double w[NS], m[6];
+    Csum = c.Ci;
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) Csum += C[k];
+    const float t = fp_to_f32(T);
+    const bool low = t <= (float)TMID;
+    double m[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) m[j] = low ? c.mi[0][j] : c.mi[1][j];
+    if (low) mix_add_r<NQ, 0>(C, m);
+    else mix_add_r<NQ, 1>(C, m);
+    if (newton_T(m, c.et, low, t, T, cv)) return true;
+    double w[NS], Ts = T, cvs = 0.0;
 #pragma unroll
     for (int k = 0; k < NQ; ++k) w[k] = C[k];
 #pragma unroll
     for (int k = NQ; k < NS; ++k) w[k] = c.Cin[k - NQ];
-    Csum = w[0];
-#pragma unroll
-    for (int k = 1; k < NS; ++k) Csum += w[k];
-    const float t = fp_to_f32(T);
-    return solve_T_from<NS, false>(w, c.et, t <= (float)TMID, t, T, m, cv);
+    const bool ok = solve_T_slow<NS, false>(w, c.et, Ts, m, cvs);
+    T = Ts;
+    cv = cvs;
+    return ok;
 }
 
 // w = dC/dt at concentrations C; T: guess in, temperature out.
@@ -364,7 +430,7 @@ __device__ __noinline__ bool rhs(const Cell<NS>& c, const double* Cin, double& T
     kin_at(T, kc);
 #pragma unroll
     for (int k = 0; k < NQ; ++k) {
-        X[k] = C[k] * kc.eg[k];
+        X[k] = k < NREF ? C[k] : C[k] * kc.eg[k];
         w[k] = 0.0;
     }
     rates<NS>(kc, C, X, Csum, w, std::make_index_sequence<NR>{});
@@ -418,14 +484,9 @@ __device__ __forceinline__ void jac(const Kin& kc, const double* C, const double
             dr1 = k * C[r0];
             fwd = dr0 * C[r0];
         }
-        double b = kc.ieg[r0];
-        if constexpr (rx.nreac == 2) b *= kc.ieg[r1 < 0 ? 0 : r1];
-        if constexpr (dn == 1) b *= kc.rt;
-        if constexpr (dn == -1) b *= kc.irt;
+        const double ikc = inv_kc_factor<R>(kc);
         double dp0, dp1 = 0.0, rev;
-        b *= kc.eg[p0];
-        if constexpr (rx.nprod == 2) b *= kc.eg[p1 < 0 ? 0 : p1];
-        b *= k;  // reverse rate constant
+        const double b = k * ikc;  // reverse rate constant
         if constexpr (rx.nprod == 1) {
             dp0 = b;
             rev = b * C[p0];
@@ -448,15 +509,10 @@ __device__ __forceinline__ void jac(const Kin& kc, const double* C, const double
         double net = 0.0, qT;
         if constexpr (bySum || rx.type != RXN_ELEMENTARY) {
             // q / k from the products, so that k = 0 needs no case of its own
-            double f = C[r0], g = kc.ieg[r0] * (kc.eg[p0] * C[p0]);
-            if constexpr (rx.nreac == 2) {
-                f *= C[r1 < 0 ? 0 : r1];
-                g *= kc.ieg[r1 < 0 ? 0 : r1];
-            }
-            if constexpr (rx.nprod == 2) g *= kc.eg[p1 < 0 ? 0 : p1] * C[p1 < 0 ? 0 : p1];
-            if constexpr (dn == 1) g *= kc.rt;
-            if constexpr (dn == -1) g *= kc.irt;
-            net = f - g;
+            double f = C[r0], g = C[p0];
+            if constexpr (rx.nreac == 2) f *= C[r1 < 0 ? 0 : r1];
+            if constexpr (rx.nprod == 2) g *= C[p1 < 0 ? 0 : p1];
+            net = fma(-ikc, g, f);
         }
         if constexpr (bySum) qT = fma(rev, hh, Tdk * net);
         else qT = fma(rev, hh, q * s);
@@ -696,6 +752,18 @@ __device__ __forceinline__ bool load(Cell<NS>& c, const double* u, double dt) {
     }
     if constexpr (NS == 10) c.Cin[0] = u[8] * INVW.v[8];
     c.Cin[NS - 1 - NQ] = rho * (1.0 - s) * INVW.v[NS - 1];
+    c.Ci = 0.0;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) c.mi[0][j] = c.mi[1][j] = 0.0;
+#pragma unroll
+    for (int k = NQ; k < NS; ++k) {
+        c.Ci += c.Cin[k - NQ];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            c.mi[0][j] = fma(c.Cin[k - NQ], D_ECOEF.c[0][k][j], c.mi[0][j]);
+            c.mi[1][j] = fma(c.Cin[k - NQ], D_ECOEF.c[1][k][j], c.mi[1][j]);
+        }
+    }
     c.T = estimate_T<NS>(u, c.et);
     c.h = 0.0;
     c.t = 0.0;

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
     // Two queues: the costly cells after the cooperative ones, then the rest.  Warps in the
     // first slot of their SM sub-partition start with the costly ones and the others with the
     // rest, so that every sub-partition gets one warp of long step chains before any gets
-    // two (a second one beside it halves both: 244 against 401 us an attempt); when there are
+    // two (a second one beside it slows both: 377 against 230 us an attempt); when there are
     // more costly cells than those warps have lanes, all warps start with them.
     const int64_t nhi = (order && coop_n) ? (int64_t)coop_n[1] : 0;
     unsigned slot;
@@ -402,14 +402,14 @@ __global__ void k_order_hist(const int32_t* __restrict__ cost, int64_t count, un
 // bins[NBIN + 1] = the cells after them in buckets from COSTLY_BUCKET up.
 // min_bucket < 0: the line with the least estimated time, the root of the sum of squares
 // (they run side by side, but slow each other) of
-//   the FP64 pipe's:  attempts of the groups / 33.8 + attempts of the lanes / 97 per us,
+//   the FP64 pipe's:  attempts of the groups / 33.8 + attempts of the lanes / 103 per us,
 //   the longest chain in a group:  73 us an attempt alone, 113 beside a second warp,
-//   the longest chain on a lane:   244 us an attempt with one warp of costly cells to a
-//                                  sub-partition and no groups, 401 beside another warp
+//   the longest chain on a lane:   230 us an attempt with one warp of costly cells to a
+//                                  sub-partition and no groups, 377 beside another warp
 // (measured, 10 species, cells of 398 attempts, 152 SMs).  A group's chain is three times
 // as fast and costs the pipe three times as much: it pays for cells far above the mean.
-constexpr float GROUP_RATE = 33.8f, LANE_RATE = 97.0f, GROUP_ALONE = 73.0f, GROUP_PAIR = 113.0f, LANE_ALONE = 244.0f,
-                LANE_PAIR = 401.0f;
+constexpr float GROUP_RATE = 33.8f, LANE_RATE = 103.0f, GROUP_ALONE = 73.0f, GROUP_PAIR = 113.0f, LANE_ALONE = 230.0f,
+                LANE_PAIR = 377.0f;
 __device__ __forceinline__ float bin_cost(int b) {  // attempts at the bin's lower edge
     return (float)(1u << (b / SUB)) * (1.0f + (float)(b % SUB) / SUB) - 1.0f;
 }

@@ -111,6 +111,15 @@ __device__ __forceinline__ void mix_coef_r(const double* w, double* m) {
         m[j] = s;
     }
 }
+// m[j] += the same sum over the first N species (moles)
+template <int N, int RG>
+__device__ __forceinline__ void mix_add_r(const double* w, double* m) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j)
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            if (D_ECOEF.c[RG][k][j] != 0.0) m[j] = fma(w[k], D_ECOEF.c[RG][k][j], m[j]);
+}
 template <int NS, bool MASS = false>
 __device__ __forceinline__ void mix_coef(const double* w, int range, double* m) {
     if (range == 0) mix_coef_r<NS, 0, MASS>(w, m);
@@ -140,7 +149,7 @@ __device__ __forceinline__ bool solve_T_any(const double* w, double et, double& 
     int range = T <= TMID ? 0 : 1;
     mix_coef<NS, MASS>(w, range, m);
     int flips = 0;
-    for (int it = 0; it < 100; ++it) {
+    for (int it = 0; it < 60; ++it) {
         const int r = T <= TMID ? 0 : 1;
         if (r != range) {
             range = r;
@@ -205,6 +214,7 @@ __device__ __forceinline__ bool newton_T(const double* m, double et, bool low, f
         fine = fabsf(dt) <= 1e-5f * t;
         if (fine || !(fabsf(dt) < 1e4f)) break;
     }
+    if (fine && t > 1.0f && t < 1e5f) T = fp_from_f32(t);  // where the iteration of any state starts
     const float edge = 0.02f;
     fine = fine && (low ? t > (float)T_LO && t < (float)TMID - edge : t > (float)TMID + edge && t < (float)T_HI);
     if (fine) {
@@ -237,7 +247,6 @@ __device__ __forceinline__ bool newton_T(const double* m, double et, bool low, f
             return true;
         }
     }
-    if (fine) T = fp_from_f32(t);
     return false;
 }
 template <int NS, bool MASS>
