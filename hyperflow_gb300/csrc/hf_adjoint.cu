@@ -249,11 +249,25 @@ __global__ void __launch_bounds__(32) k_chem_adjoint(AdjointArgs a) {
     int n_ign = -1, n_pmax = 0;
     double Ta = 0.0, Tb = 0.0, pmax = pr.p, Tprev = T0, yend = 0.0;
     unsigned long long steps = 0;
+    // BACKWARD: the last segment (from call nlast on) is recorded here already
+    const int nlast = (a.ncalls - 1) / a.K * a.K;
+    int nrec_last = 0;
     for (int n = 0; n < a.ncalls && __any_sync(grp8::FULL, live); ++n) {
         if (a.ckpt && n % a.K == 0 && live) put(a.ckpt + (int64_t)(n / a.K) * NV * cst, u);
-        int nrec = 0;
+        const bool record = BACKWARD && n >= nlast;
+        if (record && n == nlast && live) put(a.seg, u);
+        const int before = nrec_last;
+        int none = 0;
         uint32_t clip = 0;
-        const int r = run_call<NS>(u, a.dt, a.rtol, a.atol, nullptr, 0, nrec, 0, clip, yend, live, fs);
+        const int r = run_call<NS>(u, a.dt, a.rtol, a.atol, record ? a.tape + i : nullptr, cst,
+                                   record ? nrec_last : none, a.cap, clip, yend, live, fs);
+        if (record && live && r == CELL_DONE) {
+            if (t == 0) {
+                a.nstep[(int64_t)(n - nlast) * cst + i] = nrec_last - before;
+                a.clipm[(int64_t)(n - nlast) * cst + i] = clip;
+            }
+            put(a.seg + (int64_t)(n - nlast + 1) * NV * cst, u);
+        }
         if (live && r != CELL_DONE) {
             fail_cell(r == CELL_MAXSTEPS ? CELL_MAXSTEPS : CELL_FAIL);
             live = false;
@@ -312,14 +326,15 @@ __global__ void __launch_bounds__(32) k_chem_adjoint(AdjointArgs a) {
             const int n0 = sg * a.K, n1 = min(n0 + a.K, a.ncalls);
             // recompute the segment: boundary states and the tape of accepted steps
             const double* c = a.ckpt + (int64_t)sg * NV * cst;
+            const bool have = sg == nseg - 1;  // by the forward pass
             __syncwarp();
-            if (ok) {
+            if (ok && !have) {
 #pragma unroll
                 for (int v = 0; v < NV; ++v) u[v] = c[v * cst + i];
                 put(a.seg, u);
             }
-            int nrec = 0;
-            for (int n = n0; n < n1 && __any_sync(grp8::FULL, ok); ++n) {
+            int nrec = have ? nrec_last : 0;
+            for (int n = n0; n < n1 && !have && __any_sync(grp8::FULL, ok); ++n) {
                 uint32_t clip = 0;
                 const int before = nrec;
                 const int r = run_call<NS>(u, a.dt, a.rtol, a.atol, a.tape + i, cst, nrec, a.cap, clip, yend, ok, fs);

@@ -262,83 +262,92 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
     if (st->abort_run) return;  // an earlier step of this device-resident run failed
     const unsigned lane = threadIdx.x & 31;
     if (dt_dev) dt = *dt_dev;  // interval from device memory (graph-captured steps)
-    // COOP: the costliest cells first, one cell per group of 8 lanes; the rest one per
-    // lane.  Without it the kernel holds no shared memory (the L1 keeps the lanes' stacks).
-    int64_t ncoop = 0;
+    unsigned slot;
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
     unsigned long long my_attempts = 0;
-    if constexpr (COOP) {
-        __shared__ grp8::Shared sh[8];
-        ncoop = (order && coop_n) ? (int64_t)*coop_n : 0;
-        if (ncoop > 0)
-            my_attempts = group_phase<NS, true>(U, cs, cell_index, order, ncoop, count, dt, dt_cell, rtol, atol, trial,
-                                                fail, h_hist, cost, st, &sh[threadIdx.x >> 3]);
-    }
     // Two queues: the costly cells after the cooperative ones, then the rest.  Warps in the
     // first slot of their SM sub-partition start with the costly ones and the others with the
     // rest, so that every sub-partition gets one warp of long step chains before any gets
     // two (a second one beside it slows both: 377 against 230 us an attempt); when there are
     // more costly cells than those warps have lanes, all warps start with them.
+    int64_t ncoop = 0;
+    if constexpr (COOP) ncoop = (order && coop_n) ? (int64_t)*coop_n : 0;
     const int64_t nhi = (order && coop_n) ? (int64_t)coop_n[1] : 0;
-    unsigned slot;
-    asm volatile("mov.u32 %0, %%warpid;" : "=r"(slot));
     bool costly = nhi > 0 && (slot < 4 || nhi > lanes_first);
     int dry = 0;  // queues found empty
-    cell::Cell<NS> c;
-    double Lu[cell::NQ * cell::NQ];
-    int64_t cell = -1;
-    bool active = false, drained = false;
-    for (;;) {
-        if (!drained) {
-            const unsigned need = __ballot_sync(0xffffffffu, !active);
-            bool none = false;
-            if (need) {
-                const int leader = __ffs(need) - 1;
-                unsigned long long base = 0;
-                if ((int)lane == leader)
-                    base = atomicAdd(costly ? &st->costly_counter : &st->counter, (unsigned long long)__popc(need));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (!active) {
-                    const int64_t q = ncoop + (costly ? 0 : nhi) + (int64_t)(base + __popc(need & ((1u << lane) - 1u)));
-                    if (q < (costly ? ncoop + nhi : count)) {
-                        const int64_t k = order ? (int64_t)order[q] : q;
-                        cell = k;
-                        double u[NS + 3];
-                        load_cell<NS>(U, cs, cell_index ? cell_index[k] : k, u);
-                        if (cell::begin_warm<NS>(c, u, dt_cell ? dt_cell[k] : dt, h_hist ? h_hist[k] : 0.0) ==
-                            CELL_CONTINUE)
-                            active = true;
-                        else
-                            report(st, fail, k, CELL_FAIL);
-                    } else {
-                        none = true;
-                    }
-                }
+    // COOP: the costliest cells one per group of 8 lanes.  Warps in the first slots take them
+    // before anything else, the others after their lane cells, unless there are more than
+    // those warps have groups.  Without COOP the kernel holds no shared memory (the L1 keeps
+    // the lanes' stacks).
+    const bool groups_first = slot < 4 || 8 * ncoop > lanes_first;
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+        if ((part == 0) == groups_first) {
+            if constexpr (COOP) {
+                __shared__ grp8::Shared sh[8];
+                if (ncoop > 0)
+                    my_attempts += group_phase<NS, true>(U, cs, cell_index, order, ncoop, count, dt, dt_cell, rtol, atol,
+                                                         trial, fail, h_hist, cost, st, &sh[threadIdx.x >> 3]);
             }
-            if (__any_sync(0xffffffffu, none)) {  // this queue is empty: the other one next
-                costly = !costly;
-                drained = ++dry == 2 || (nhi == 0 && dry == 1);
-            }
-        }
-        if (!__any_sync(0xffffffffu, active)) {
-            if (drained) break;
             continue;
         }
-        if (active) {
-            bool screened = false;
-            const int r = cell::attempt<NS, true, 1>(c, rtol, atol, Lu, &screened);
-            if (r != CELL_CONTINUE) {
-                my_attempts += c.attempts;
-                double u[NS + 3];
-                if (r == CELL_DONE && cell::finish<NS>(c, u)) {
-#pragma unroll
-                    for (int n = 0; n < NS + 3; ++n) trial[n * count + cell] = u[n];
-                    fail[cell] = 0;
-                    if (h_hist && !screened) h_hist[cell] = c.h;
-                    if (cost) cost[cell] = c.attempts;
-                } else {
-                    report(st, fail, cell, r == CELL_MAXSTEPS ? CELL_MAXSTEPS : CELL_FAIL);
+        cell::Cell<NS> c;
+        double Lu[cell::NQ * cell::NQ];
+        int64_t cell = -1;
+        bool active = false, drained = false;
+        for (;;) {
+            if (!drained) {
+                const unsigned need = __ballot_sync(0xffffffffu, !active);
+                bool none = false;
+                if (need) {
+                    const int leader = __ffs(need) - 1;
+                    unsigned long long base = 0;
+                    if ((int)lane == leader)
+                        base = atomicAdd(costly ? &st->costly_counter : &st->counter, (unsigned long long)__popc(need));
+                    base = __shfl_sync(0xffffffffu, base, leader);
+                    if (!active) {
+                        const int64_t q = ncoop + (costly ? 0 : nhi) + (int64_t)(base + __popc(need & ((1u << lane) - 1u)));
+                        if (q < (costly ? ncoop + nhi : count)) {
+                            const int64_t k = order ? (int64_t)order[q] : q;
+                            cell = k;
+                            double u[NS + 3];
+                            load_cell<NS>(U, cs, cell_index ? cell_index[k] : k, u);
+                            if (cell::begin_warm<NS>(c, u, dt_cell ? dt_cell[k] : dt, h_hist ? h_hist[k] : 0.0) ==
+                                CELL_CONTINUE)
+                                active = true;
+                            else
+                                report(st, fail, k, CELL_FAIL);
+                        } else {
+                            none = true;
+                        }
+                    }
                 }
-                active = false;
+                if (__any_sync(0xffffffffu, none)) {  // this queue is empty: the other one next
+                    costly = !costly;
+                    drained = ++dry == 2 || (nhi == 0 && dry == 1);
+                }
+            }
+            if (!__any_sync(0xffffffffu, active)) {
+                if (drained) break;
+                continue;
+            }
+            if (active) {
+                bool screened = false;
+                const int r = cell::attempt<NS, true, 1>(c, rtol, atol, Lu, &screened);
+                if (r != CELL_CONTINUE) {
+                    my_attempts += c.attempts;
+                    double u[NS + 3];
+                    if (r == CELL_DONE && cell::finish<NS>(c, u)) {
+#pragma unroll
+                        for (int n = 0; n < NS + 3; ++n) trial[n * count + cell] = u[n];
+                        fail[cell] = 0;
+                        if (h_hist && !screened) h_hist[cell] = c.h;
+                        if (cost) cost[cell] = c.attempts;
+                    } else {
+                        report(st, fail, cell, r == CELL_MAXSTEPS ? CELL_MAXSTEPS : CELL_FAIL);
+                    }
+                    active = false;
+                }
             }
         }
     }

@@ -28,8 +28,16 @@ struct Slot {
     double b, E, b0, E0, lfc;
     int r0, r1, p0, p1;  // species, -1 none
     int dn, type, third; // third: 1 + efficiency set, 0 none
+    int low;             // falloff: the lane whose last slot is its k0; extra slots: the reaction
     int dup;             // 1: add the next slot's rate constant (same species); -1: added there
 };
+// Slots NR, NR + 1, ... (idle otherwise) evaluate the low-pressure rate constants of the
+// falloff reactions, in one round with the others' exponentials.
+constexpr int fall_reaction(int f) {
+    for (int r = 0; r < NR; ++r)
+        if (RXN[r].type == RXN_FALLOFF && fall_index(r) == f) return r;
+    return -1;
+}
 constexpr int NEFF = 2, NVAL = 5;  // per slot: dq/dC of the four participants, dq/dM
 constexpr int MAXLIST = 20;
 struct Tables {
@@ -48,13 +56,21 @@ struct Tables {
 };
 constexpr Tables make_tables() {
     Tables t{};
-    t.ok = NR <= NSLOT;
+    t.ok = NR + NFALL <= NSLOT && NR / G == NROUND - 1;  // the extra slots are in the last round
     const cell::NetNu nu = cell::make_nu();
     for (int r = 0; r < NSLOT; ++r) {
         Slot& s = t.s[r];
         s.r0 = s.r1 = s.p0 = s.p1 = -1;
-        if (r >= NR) continue;
+        if (r >= NR) {
+            if (r < NR + NFALL) {
+                s.b = RXN[fall_reaction(r - NR)].b0;
+                s.E = RXN[fall_reaction(r - NR)].Ea0R;
+                s.low = fall_reaction(r - NR);
+            }
+            continue;
+        }
         const Reaction& x = RXN[r];
+        s.low = x.type == RXN_FALLOFF ? (NR + fall_index(r)) % G : 0;
         s.b = x.b; s.E = x.EaR; s.b0 = x.b0; s.E0 = x.Ea0R;
         s.type = x.type;
         s.lfc = x.type == RXN_FALLOFF ? const_log10(x.troeA) : 0.0;
@@ -265,10 +281,9 @@ __device__ __forceinline__ void kin_at(double T, Kin& k) {
 
 // Falloff factor of the lanes whose slot is one (hf_cell.cuh falloff, data-driven).
 template <bool JAC>
-__device__ __forceinline__ double falloff(const Slot& s, const Kin& kc, double kinf, double A0, double M, double& Tdk,
+__device__ __forceinline__ double falloff(const Slot& s, const Kin& kc, double kinf, double k0, double M, double& Tdk,
                                           double& dkM) {
-    const double lFc = s.lfc, c = fma(-0.67, lFc, -0.4), nn = fma(-1.27, lFc, 0.75);
-    const double k0 = A0 * cell::fexp(fma(s.b0, kc.lnT, -s.E0 * kc.invT)), k0M = k0 * M;
+    const double lFc = s.lfc, c = fma(-0.67, lFc, -0.4), nn = fma(-1.27, lFc, 0.75), k0M = k0 * M;
     const double Pr = fp_div(k0M, kinf);
     const bool tiny = !(__double2hiint(Pr) >= 0x01a56e1f);
     const double x = fma(cell::flog(tiny ? 1e-300 : Pr), fm::INV_LN10, c);
@@ -290,21 +305,25 @@ __device__ __forceinline__ double falloff(const Slot& s, const Kin& kc, double k
 
 // The lane's reactions into shared memory: q, and with JAC also T dq/dT, the partials and
 // (where qo is given) the rates of progress with the slots' own rate constants.
+// klast: in and out, the rate constant of the lane's slot of the last round (taken first).
 template <int rnd, bool JAC>
 __device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X, double M1, double M2, Shared* sh,
-                                               double* qo) {
+                                               double* qo, double& klast) {
     const int t = lane8();
     {
         const int r = rnd * G + t;
         const Slot& s = D_TAB.s[r];
-        const double A = r < NR ? c_A[r] : 0.0;
+        double A = r < NR ? c_A[r] : 0.0;
+        if constexpr (rnd == NROUND - 1) A = r >= NR && r < NR + NFALL ? c_A0[s.low] : A;
         double k = A * cell::fexp(fma(s.b, kc.lnT, -s.E * kc.invT));
         double Tdk = 0.0, dkM = 0.0;
+        if constexpr (rnd == NROUND - 1) klast = k;
         if constexpr (JAC) Tdk = k * fma(s.E, kc.invT, s.b);
         if constexpr (round_has_third(rnd)) {
             const double M = s.third == 2 ? M2 : M1;
+            const double k0 = get(klast, s.low & 7);
             if (s.type == RXN_FALLOFF) {
-                k = falloff<JAC>(s, kc, k, c_A0[r < NR ? r : 0], M, Tdk, dkM);
+                k = falloff<JAC>(s, kc, k, k0, M, Tdk, dkM);
             } else if (s.type == RXN_THREE_BODY) {
                 dkM = k;
                 k *= M;
@@ -363,9 +382,10 @@ __device__ __forceinline__ void reactions(const Kin& kc, double C, double M1, do
                                           double* qo = nullptr) {
     static_assert(NROUND == 3, "three rounds of reactions");
     const double X = C * kc.eg;
-    reaction_round<0, JAC>(kc, C, X, M1, M2, sh, qo);
-    reaction_round<1, JAC>(kc, C, X, M1, M2, sh, qo);
-    reaction_round<2, JAC>(kc, C, X, M1, M2, sh, qo);
+    double klast = 0.0;
+    reaction_round<2, JAC>(kc, C, X, M1, M2, sh, qo, klast);
+    reaction_round<0, JAC>(kc, C, X, M1, M2, sh, qo, klast);
+    reaction_round<1, JAC>(kc, C, X, M1, M2, sh, qo, klast);
 }
 
 struct RhsOut {
