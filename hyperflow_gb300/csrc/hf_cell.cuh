@@ -15,7 +15,7 @@
 //    prod_prod exp(g), q = k (prod_reac C - prod_reac exp(-g) prod_prod X).
 //  * Reactions that differ only in k (the duplicate pairs) are evaluated once.
 //  * g = h/RT - s/R by one polynomial; exponentials and logarithms from larger tables
-//    (below); one second-order FP64 Newton step for T (solve_T_from).
+//    (below); one second-order FP64 Newton step for T (newton_T).
 //  * Jacobian, LU factorisation and the frozen-cell screen are one function, so J never
 //    leaves the registers; every attempt starts with it.  A rejected step evaluates J
 //    again, which costs nothing: the lanes of its warp that accepted theirs, or hold a new

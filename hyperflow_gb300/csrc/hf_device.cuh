@@ -185,19 +185,15 @@ __device__ __noinline__ bool solve_T_slow(const double* w, double et, double& T,
     return true;
 }
 
-// Solves e(T) = R et for the weights w (moles, or with MASS partial densities): T, the
-// FP64 mixture coefficients m of its range and the heat capacity cv = poly_cv(m, T).  T on
-// entry starts the iteration of states that need solve_T_any.
-//
-// FP64 instructions are what this costs, so one FP64 Newton step of second order replaces
-// the iteration to 1e-10: e(T0) against its values at T_LO, T_MID and T_HI in FP32 picks
-// the range and a secant guess t (solve_T_from takes both from its caller), FP32 Newton
-// steps converge to FP32 accuracy (T within about 1e-6), and with r = et - e(T0) the FP64
-// step
+// The fast solve of e(T) = R et: newton_T from the FP64 mixture coefficients m of the range
+// that holds T, giving T and the heat capacity cv = poly_cv(m, T).  FP64 instructions are
+// what a solve costs, so one FP64 Newton step of second order replaces the iteration to
+// 1e-10: secant_T compares et with e at T_LO, T_MID and T_HI in FP32 for the range and a
+// guess t (the chemistry has both from the step before), FP32 Newton steps converge to FP32
+// accuracy (T within about 1e-6), and with r = et - e(T0) the FP64 step
 //     T = T0 + d - (cv'/2cv) d^2,  d = r / cv
 // leaves an error of order (d/T)^3, below rounding for d <= 4e-6 T.  The mixture
-// coefficients (a sum over species for each power of T) are most of what is left: 90 FP64
-// instructions a solve.  States near T_mid, outside [T_LO, T_HI], or whose FP32 phase does
+// coefficients (a sum over species for each power of T) are most of what is left.  States near T_mid, outside [T_LO, T_HI], or whose FP32 phase does
 // not settle take solve_T_any.
 //
 // newton_T: the Newton steps from mixture coefficients m of the range `low` names; false
@@ -250,41 +246,18 @@ __device__ __forceinline__ bool newton_T(const double* m, double et, bool low, f
     return false;
 }
 template <int NS, bool MASS>
-__device__ __forceinline__ bool solve_T_from(const double* w, double et, bool low, float t, double& T, double* m,
-                                             double& cv) {
-    if (low) mix_coef_r<NS, 0, MASS>(w, m);
-    else mix_coef_r<NS, 1, MASS>(w, m);
-    if (newton_T(m, et, low, t, T, cv)) return true;
-    // through copies, so that the arrays of the fast path stay in registers
-    double ws[NS], ms[6], Ts = T, cvs = 0.0;
+__device__ __forceinline__ void secant_T(const double* w, float et, bool& low, float& t) {
+    float lo = 0.0f, mid = 0.0f, hi = 0.0f;
 #pragma unroll
-    for (int k = 0; k < NS; ++k) ws[k] = w[k];
-    const bool ok = solve_T_slow<NS, MASS>(ws, et, Ts, ms, cvs);
-#pragma unroll
-    for (int j = 0; j < 6; ++j) m[j] = ms[j];
-    T = Ts;
-    cv = cvs;
-    return ok;
-}
-template <int NS, bool MASS = false>
-__device__ __forceinline__ bool solve_T(const double* w, double et, double& T, double* m, double& cv) {
-    float t;
-    const float etf = fp_to_f32(et);
-    bool low;
-    {
-        float lo = 0.0f, mid = 0.0f, hi = 0.0f;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            const float f = fp_to_f32(w[k]);
-            lo = fmaf(f, (float)(MASS ? D_EAT_MASS.lo[k] : D_EAT.lo[k]), lo);
-            mid = fmaf(f, (float)(MASS ? D_EAT_MASS.mid[k] : D_EAT.mid[k]), mid);
-            hi = fmaf(f, (float)(MASS ? D_EAT_MASS.hi[k] : D_EAT.hi[k]), hi);
-        }
-        low = etf <= mid;
-        t = low ? (float)T_LO + (etf - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
-                : (float)TMID + (etf - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
+    for (int k = 0; k < NS; ++k) {
+        const float f = fp_to_f32(w[k]);
+        lo = fmaf(f, (float)(MASS ? D_EAT_MASS.lo[k] : D_EAT.lo[k]), lo);
+        mid = fmaf(f, (float)(MASS ? D_EAT_MASS.mid[k] : D_EAT.mid[k]), mid);
+        hi = fmaf(f, (float)(MASS ? D_EAT_MASS.hi[k] : D_EAT.hi[k]), hi);
     }
-    return solve_T_from<NS, MASS>(w, et, low, t, T, m, cv);
+    low = et <= mid;
+    t = low ? (float)T_LO + (et - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
+            : (float)TMID + (et - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
 }
 
 // The same for a specific energy e (J/kg) and weights z_k = Y_k / W_k, from a warm guess:
@@ -348,20 +321,63 @@ __device__ __forceinline__ bool state_ok(const double* q, double rho) {
 // solve that fails).  T_guess seeds the UV inversion.  In units of volume: with
 // M_j = sum_k q_k c_kj / W_k the energy equation is sum_j M_j T^(j+1) + M_5 =
 // (E - |m|^2 / 2 rho) / R, so no mass fractions are formed.
+// Species whose partial density is below 2^-110 of the largest add less than 2^-98 of the
+// largest term of any sum formed here (the coefficients' ratios stay below 2^12): no sum
+// changes by a bit unless its terms cancel to 2^-45, so a warp in which all lanes agree on
+// it leaves such species out.  In unburnt gas that is 7 of 10, and a solve takes 58 FP64
+// instructions instead of 114.
+template <int NS>
+__device__ __forceinline__ unsigned live_species(const double* q) {
+    unsigned top = 0, live = 0;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) top = max(top, fp_abs_hi(q[k]));
+#pragma unroll
+    for (int k = 0; k < NS; ++k) live |= (fp_abs_hi(q[k]) + 0x06e00000u >= top ? 1u : 0u) << k;
+    return __reduce_or_sync(__activemask(), live);
+}
+template <int NS, int RG>
+__device__ __forceinline__ void mix_live(const double* q, unsigned live, double* m) {
+#pragma unroll
+    for (int j = 0; j < 6; ++j) m[j] = 0.0;
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+        if (live >> k & 1u) {
+#pragma unroll
+            for (int j = 0; j < 6; ++j)
+                if (D_ECOEF_MASS.c[RG][k][j] != 0.0) m[j] = fma(q[k], D_ECOEF_MASS.c[RG][k][j], m[j]);
+        }
+}
 template <int NS>
 __device__ __forceinline__ bool properties(const double* q, Props& s, double T_guess, Prim& pr) {
-    double rho = q[0];
+    const unsigned live = live_species<NS>(q);
+    double rho = 0.0, zs = 0.0;  // zs = sum_k q_k / W_k
 #pragma unroll
-    for (int k = 1; k < NS; ++k) rho += q[k];
+    for (int k = 0; k < NS; ++k)
+        if (live >> k & 1u) {
+            rho += q[k];
+            zs = fma(q[k], INVW.v[k], zs);
+        }
     if (!state_ok<NS>(q, rho)) return false;
     const double ir = fp_rcp(rho);
-    double zs = 0.0;  // sum_k q_k / W_k
-#pragma unroll
-    for (int k = 0; k < NS; ++k) zs = k ? fma(q[k], INVW.v[k], zs) : q[k] * INVW.v[k];
     const double ke = fma(q[NS], q[NS], q[NS + 1] * q[NS + 1]) * ir;
     const double et = fma(-0.5, ke, q[NS + 2]) * (1.0 / RU);
     double T = T_guess, m[6], cv;
-    if (!solve_T<NS, true>(q, et, T, m, cv)) return false;
+    {
+        float t;
+        bool low;
+        secant_T<NS, true>(q, fp_to_f32(et), low, t);
+        if (low) mix_live<NS, 0>(q, live, m);
+        else mix_live<NS, 1>(q, live, m);
+        if (!newton_T(m, et, low, t, T, cv)) {
+            // through copies, so that the arrays of the fast path stay in registers
+            double ws[NS], Ts = T, cvs = 0.0;
+#pragma unroll
+            for (int k = 0; k < NS; ++k) ws[k] = q[k];
+            if (!solve_T_slow<NS, true>(ws, et, Ts, m, cvs)) return false;
+            T = Ts;
+            cv = cvs;
+        }
+    }
     pr.rho = rho;
     pr.ir = ir;
     s.T = T;
@@ -387,17 +403,9 @@ __device__ __forceinline__ bool properties(const double* q, Props& s, double T_g
 // A temperature of the state q near its own (secants of e(T) in FP32), to start a solve.
 template <int NS>
 __device__ __forceinline__ double estimate_T(const double* q, double et) {
-    float lo = 0.0f, mid = 0.0f, hi = 0.0f;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-        const float f = fp_to_f32(q[k]);
-        lo = fmaf(f, (float)D_EAT_MASS.lo[k], lo);
-        mid = fmaf(f, (float)D_EAT_MASS.mid[k], mid);
-        hi = fmaf(f, (float)D_EAT_MASS.hi[k], hi);
-    }
-    const float e = fp_to_f32(et);
-    const float t = e <= mid ? (float)T_LO + (e - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
-                             : (float)TMID + (e - mid) * ((float)(T_HI - TMID) * fp_rcp_seed(hi - mid));
+    float t;
+    bool low;
+    secant_T<NS, true>(q, fp_to_f32(et), low, t);
     return t > 50.0f && t < 9000.0f ? fp_from_f32(t) : 1000.0;
 }
 
