@@ -136,7 +136,11 @@ __global__ void k_fill(Level L, const hf_patch* __restrict__ patches, int npatch
             const hf_patch& Q = patches[q];
             if (wi >= Q.ilo && wi < Q.ilo + Q.nx && wj >= Q.jlo && wj < Q.jlo + Q.ny) {
                 GView s{U, Q};
-                for (int n = 0; n < NS + 3; ++n) v.at(gi, gj, n) = s.at(wi, wj, n);
+                double val[NS + 3];
+#pragma unroll
+                for (int n = 0; n < NS + 3; ++n) val[n] = s.at(wi, wj, n);
+#pragma unroll
+                for (int n = 0; n < NS + 3; ++n) v.at(gi, gj, n) = val[n];
                 return;
             }
         }
@@ -895,9 +899,15 @@ __device__ __forceinline__ void interp_one(const hf_patch& C, const double* __re
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
         q[n] = rd(ci, cj, n);
-        sx[n] = minmod(q[n] - rd(ci - 1, cj, n), rd(ci + 1, cj, n) - q[n]);
-        sy[n] = minmod(q[n] - rd(ci, cj - 1, n), rd(ci, cj + 1, n) - q[n]);
+        const double x = 0.25 * minmod(q[n] - rd(ci - 1, cj, n), rd(ci + 1, cj, n) - q[n]);
+        const double y = 0.25 * minmod(q[n] - rd(ci, cj - 1, n), rd(ci, cj + 1, n) - q[n]);
+        sx[n] = x + y;  // the child at (1, 1), less at (0, 0); sy: at (1, 0), less at (0, 1)
+        sy[n] = x - y;
     }
+    // value of child (a, b): one product and sum per component
+    auto child_value = [&](int a, int b, double theta, int n) {
+        return a == b ? fma(a ? theta : -theta, sx[n], q[n]) : fma(a ? theta : -theta, sy[n], q[n]);
+    };
     double theta = 1.0;
     bool accepted = false;
     for (int attempt = 0; attempt < 48; ++attempt) {
@@ -906,7 +916,7 @@ __device__ __forceinline__ void interp_one(const hf_patch& C, const double* __re
             for (int a = 0; a < 2 && good; ++a) {
                 double child[NV];
 #pragma unroll
-                for (int n = 0; n < NV; ++n) child[n] = q[n] + theta * ((a ? 0.25 : -0.25) * sx[n] + (b ? 0.25 : -0.25) * sy[n]);
+                for (int n = 0; n < NV; ++n) child[n] = child_value(a, b, theta, n);
                 good = admissible_state<NS>(child, 0.0);
             }
         if (good) { accepted = true; break; }
@@ -920,7 +930,7 @@ __device__ __forceinline__ void interp_one(const hf_patch& C, const double* __re
 #pragma unroll
             for (int n = 0; n < NV; ++n)
                 Uf[F.offset + (int64_t)n * F.comp_stride + (int64_t)(fj - F.jlo + F.ng) * F.pitch + (fi - F.ilo + F.ng)] =
-                    q[n] + theta * ((a ? 0.25 : -0.25) * sx[n] + (b ? 0.25 : -0.25) * sy[n]);
+                    child_value(a, b, theta, n);
         }
 }
 template <int NS>
