@@ -1,8 +1,8 @@
 // Discrete adjoint of the chemistry calls (a build-defined extension: the
 // reference has no sensitivity code).  A 0D cell at constant (rho, e) is advanced
 // by ncalls chemistry calls of dt each, every call exactly as Chemistry::advance
-// (HyperFlow_V3/src/chemistry.cpp:55-76, here the plain Rodas4 integration of
-// hf_kinetics.cuh: adaptive steps, clip y >= -1e-13 to 0, last species closes the
+// (HyperFlow_V3/src/chemistry.cpp:55-76, here the Rodas4 integration of
+// hf_group.cuh: adaptive steps, clip y >= -1e-13 to 0, last species closes the
 // mass).  An objective J of the temperatures / pressures at the call boundaries
 // is differentiated with respect to p_r = ln(multiplier_r) of every reaction
 // (the multiplier scales the forward and reverse rate constants; for falloff
@@ -206,7 +206,7 @@ enum { OBJ_IGNITION = HF_OBJ_IGNITION_DELAY, OBJ_PEAK_PRESSURE = HF_OBJ_PEAK_PRE
 // Forward pass: ncalls calls with checkpoints (ckpt may be null), objective
 // bookkeeping; then (BACKWARD) the reverse sweep.  One cell per group of 8 lanes, four per
 // warp and block: the cells' step chains are what a run waits for (1,024 cells, 8 calls and
-// their reverse: 1,030 ms with one cell per lane).  The forward-only instantiation carries
+// their reverse: 155 ms, 1,236 with one cell per lane).  The forward-only instantiation carries
 // none of the reverse sweep's registers.
 #pragma nv_diag_suppress 128  // the forward-only instantiation ends before the reverse sweep's loops
 template <int NS, bool BACKWARD>
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(32) k_chem_adjoint(AdjointArgs a) {
     __shared__ Sh shm[4];
     Sh* const sh = &shm[threadIdx.x >> 3];
     grp8::Shared* fs;
-    if constexpr (BACKWARD) fs = &sh->st[0].s;
+    if constexpr (BACKWARD) fs = &sh->f;
     else fs = sh;
     const int t = grp8::lane8();
     const int64_t want = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 3);
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(32) k_chem_call_adjoint(hf_patch P, const doub
     int nrec = 0;
     uint32_t clip = 0;
     double yend = 0.0;
-    const int r = run_call<NS>(uc, dt, rtol, atol, tape + li, chunk, nrec, cap, clip, yend, live, &sh->st[0].s);
+    const int r = run_call<NS>(uc, dt, rtol, atol, tape + li, chunk, nrec, cap, clip, yend, live, &sh->f);
     bool ok = live && r == CELL_DONE && nrec <= cap;
     const Interval<NS> v = interval<NS>(u);
     const double mx = u[NS], my = u[NS + 1], E = u[NS + 2], ir = v.ir;

@@ -2,11 +2,12 @@
 // with the 8 reacting species (H2, O2, H2O, H, O, OH, HO2, H2O2) spread over a group's lanes.
 //
 // Why: a warp's FP64 instruction holds its sub-partition for 64 cycles whatever the number
-// of active lanes, so one cell's step chain (about 5,500 FP64 instructions an attempt on one
+// of active lanes, so one cell's step chain (about 5,100 FP64 instructions an attempt on one
 // lane) is what a batch waits for once its expensive cells no longer fill the 608
 // sub-partitions.  Here lane t holds species t, row t of the matrix and of its LU factors
-// and evaluates reactions t, t + 8, t + 16: about 1,600 FP64 instructions an attempt, at
-// 2.3 times the instructions per cell.  All four groups of a warp run the same
+// and evaluates reactions t, t + 8, t + 16: about 1,600 FP64 instructions an attempt:
+// 73 us alone on its sub-partition against 206 on a lane, at about 3 times the pipe's time per
+// cell once the chip is full (rates measured at k_order_scan, hf_chem.cu).  All four groups of a warp run the same
 // instructions; groups without a cell, or whose step already failed, compute along on valid
 // numbers and write nothing, so no shuffle is ever divergent.
 //
@@ -205,8 +206,12 @@ __device__ __forceinline__ double reduce_scatter(const double (&v)[G]) {
     return keep + __shfl_xor_sync(FULL, send, 1);
 }
 
+struct Partials {  // of one group's reactions: T dq/dT, and per reaction the NVAL partials
+    double qT[NR], v[NR * NVAL];
+};
 struct Shared {  // of one group
-    double q[NSLOT], qT[NSLOT], v[NSLOT * NVAL];
+    double q[NR];
+    Partials p;
 };
 
 // A group's cell; every lane holds the same values but for y (mass fraction of its species).
@@ -303,15 +308,16 @@ __device__ __forceinline__ double falloff(const Slot& s, const Kin& kc, double k
     return k;
 }
 
-// The lane's reactions into shared memory: q, and with JAC also T dq/dT, the partials and
+// The lane's reactions into shared memory: q, and with JAC also T dq/dT, the partials (p) and
 // (where qo is given) the rates of progress with the slots' own rate constants.
 // klast: in and out, the rate constant of the lane's slot of the last round (taken first).
 template <int rnd, bool JAC>
-__device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X, double M1, double M2, Shared* sh,
-                                               double* qo, double& klast) {
+__device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X, double M1, double M2, double* q,
+                                               Partials* p, double* qo, double& klast) {
     const int t = lane8();
     {
         const int r = rnd * G + t;
+        const bool in = rnd < NROUND - 1 || r < NR;  // the slots past the reactions write nothing
         const Slot& s = D_TAB.s[r];
         double A = r < NR ? c_A[r] : 0.0;
         if constexpr (rnd == NROUND - 1) A = r >= NR && r < NR + NFALL ? c_A0[s.low] : A;
@@ -350,7 +356,7 @@ __device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X
             const double Xc = get(X, i2);
             double Xd = get(X, i3);
             Xd = s.p1 < 0 ? 1.0 : Xd;
-            sh->q[r] = k * fma(-(b * Xc), Xd, Ca * Cb);
+            if (in) q[r] = k * fma(-(b * Xc), Xd, Ca * Cb);
         } else {
             const double Cc = get(C, i2), ec = get(kc.eg, i2);
             double Cd = get(C, i3), ed = get(kc.eg, i3);
@@ -364,28 +370,31 @@ __device__ __forceinline__ void reaction_round(const Kin& kc, double C, double X
             hd = s.p1 < 0 ? 0.0 : hd;
             double hh = (hc + hd) - (ha + hb);
             if constexpr (round_has_dn(rnd)) hh -= s.dn == 1 ? 1.0 : s.dn == -1 ? -1.0 : 0.0;
-            sh->q[r] = k * net;
-            if (qo) qo[r] = own * net;
-            sh->qT[r] = fma(kr * cc, hh, Tdk * net);
-            double* v = sh->v + r * NVAL;
-            v[0] = k * Cb;
-            v[1] = k * Ca;
-            v[2] = kr * Cd;
-            v[3] = kr * Cc;
-            v[4] = 0.0;
-            if constexpr (round_has_third(rnd)) v[4] = dkM * net;
+            const double own_q = own * net;
+            if (in) {
+                q[r] = k * net;
+                if (qo) qo[r] = own_q;
+                p->qT[r] = fma(kr * cc, hh, Tdk * net);
+                double* v = p->v + r * NVAL;
+                v[0] = k * Cb;
+                v[1] = k * Ca;
+                v[2] = kr * Cd;
+                v[3] = kr * Cc;
+                v[4] = 0.0;
+                if constexpr (round_has_third(rnd)) v[4] = dkM * net;
+            }
         }
     }
 }
 template <bool JAC>
-__device__ __forceinline__ void reactions(const Kin& kc, double C, double M1, double M2, Shared* sh,
-                                          double* qo = nullptr) {
+__device__ __forceinline__ void reactions(const Kin& kc, double C, double M1, double M2, double* q,
+                                          Partials* p, double* qo = nullptr) {
     static_assert(NROUND == 3, "three rounds of reactions");
     const double X = C * kc.eg;
     double klast = 0.0;
-    reaction_round<2, JAC>(kc, C, X, M1, M2, sh, qo, klast);
-    reaction_round<0, JAC>(kc, C, X, M1, M2, sh, qo, klast);
-    reaction_round<1, JAC>(kc, C, X, M1, M2, sh, qo, klast);
+    reaction_round<2, JAC>(kc, C, X, M1, M2, q, p, qo, klast);
+    reaction_round<0, JAC>(kc, C, X, M1, M2, q, p, qo, klast);
+    reaction_round<1, JAC>(kc, C, X, M1, M2, q, p, qo, klast);
 }
 
 struct RhsOut {
@@ -402,7 +411,7 @@ __device__ __noinline__ RhsOut rhs(double C, double T, double et, double Ci0, do
     o.T = T;
     Kin kc;
     kin_at<false>(T, kc);
-    reactions<false>(kc, C, M1, M2, sh);
+    reactions<false>(kc, C, M1, M2, sh->q, &sh->p);
     __syncwarp();
     const int t = lane8();
     double w = 0.0;
@@ -425,7 +434,7 @@ __device__ __noinline__ RhsOut rhs_jac(double C, double T, double et, double Ci0
     o.T = T;
     Kin kc;
     kin_at<true>(T, kc);
-    reactions<true>(kc, C, M1, M2, sh);
+    reactions<true>(kc, C, M1, M2, sh->q, &sh->p);
     __syncwarp();
     const int t = lane8();
     double w = 0.0, wT = 0.0, wM = 0.0;
@@ -434,8 +443,8 @@ __device__ __noinline__ RhsOut rhs_jac(double C, double T, double et, double Ci0
         const int r = D_TAB.wr[t][e];
         const double n = D_TAB.wn[t][e];
         w = fma(n, sh->q[r], w);
-        wT = fma(n, sh->qT[r], wT);
-        wM = fma(n, sh->v[r * NVAL + 4], wM);
+        wT = fma(n, sh->p.qT[r], wT);
+        wM = fma(n, sh->p.v[r * NVAL + 4], wM);
     }
     const double tau = (1.0 - kc.h) * fp_rcp(cv);
     double a[NQ];
@@ -443,7 +452,7 @@ __device__ __noinline__ RhsOut rhs_jac(double C, double T, double et, double Ci0
     for (int j = 0; j < NQ; ++j) {
         double s = fma(wT, get(tau, j), wM);
 #pragma unroll
-        for (int e = D_TAB.j0[j]; e < D_TAB.j0[j + 1]; ++e) s = fma(D_TAB.jn[t][e], sh->v[D_TAB.jr[t][e]], s);
+        for (int e = D_TAB.j0[j]; e < D_TAB.j0[j + 1]; ++e) s = fma(D_TAB.jn[t][e], sh->p.v[D_TAB.jr[t][e]], s);
         a[j] = s;
     }
     __syncwarp();
