@@ -35,16 +35,21 @@ sys.path.insert(0, ROOT)
 METRIC = "cell-steps/s, 2D H2 detonation FP64: batched vs plain GPU; adjoint/forward time"
 NX, NY = 2048, 512
 STRIP_ROWS = 32  # rows of the periodic strip the CPU legs time
-# From one ncu capture of the probe launch below at the full size (2048 x 512, the state
-# after the 3 warm-up and 8 timed steps; `bench.py --probe-only --warmup 11`, the second
-# k_chem_batched launch of the probe, 1,090,021 step attempts, k_chem_batched<10, 4, 0>):
+# From ncu captures of the probe launch below (the state after the 3 warm-up and 8 timed
+# steps; `bench.py --probe-only --warmup 11`, the second k_chem_batched launch of the probe):
 # * FP64 flops per integrator step attempt (DFMA x 2 + DADD + DMUL thread instructions
-#   over the launch's attempts; the screened cells' kinetics pass is included), the
-#   executed-flop figure beside the algorithmic one;
-# * DRAM bytes of that launch (dram__bytes_read.sum + dram__bytes_write.sum): mostly the
-#   lanes' stack frames written back from L2.
-EXECUTED_FLOPS_PER_ATTEMPT = 2.063e4
-PROBE_TRAFFIC = 5011249000
+#   over the launch's 272,755 attempts on 512 x 128 cells; the cells in groups of 8 lanes
+#   included), the executed-flop figure beside the algorithmic one;
+# * DRAM bytes of the launch at the full size (2048 x 512, 1,090,021 attempts;
+#   dram__bytes_read.sum + dram__bytes_write.sum): mostly the lanes' stack frames written
+#   back from L2;
+# * the FP64 pipe's active share of the full-size launch's cycles.
+EXECUTED_FLOPS_PER_ATTEMPT = 1.237e4
+PROBE_TRAFFIC = 1966000000
+PROBE_FP64_PIPE = 0.809
+# FP64-pipe instructions per cell-step of the flux path, per lane (ncu counts of one x-face,
+# y-face, update and CFL launch of the same run on 512 x 128 cells: 311, 305, 52 and 91 each)
+FLUX_FP64_PER_CELL_STEP = 4 * (311 + 305 + 52) + 91
 # algorithmic HBM bytes of one cell-step (NS = 10): 4 Euler stages reading U (and U_old in
 # the Heun stages) and writing U, plus chemistry reading and writing U
 BYTES_PER_CELL_STEP = 1248
@@ -190,7 +195,13 @@ def flux_roofline(ff, nv, cells, flux_ms_per_step, fp64_peak, hbm_gbs):
     return {"kernels": "k_face_plain (x, y) + k_update_plain, k_fill, k_cfl of a step",
             "bound": "fp64" if gf / fp64_peak >= gb / hbm_gbs else "hbm", "ms_per_step": flux_ms_per_step,
             "fp64": {"flops_per_cell_step": flops, "achieved": gf, "peak": fp64_peak, "unit": "GFLOP/s",
-                     "frac": gf / fp64_peak, "per_face": ff["face"], "per_cell_update": ff["cell"],
+                     "frac": gf / fp64_peak,
+                     "executed": {"instructions_per_cell_step": FLUX_FP64_PER_CELL_STEP,
+                                  "frac": FLUX_FP64_PER_CELL_STEP * cells / sec / (0.5e9 * fp64_peak),
+                                  "note": "FP64-pipe instructions the path runs (ncu, 512 x 128 cells) against the "
+                                          "pipe's instruction rate; frac above counts the oracle's formulation, "
+                                          "which needs more"},
+                     "per_face": ff["face"], "per_cell_update": ff["cell"],
                      "per_combine": ff["combine"],
                      "source": "the oracle's flux functions on a counting scalar, 3 UV Newton iterations per "
                                "EOS solve from 1000 K, at a subsonic face of the fresh gas (HLLC star state)"},
@@ -731,8 +742,10 @@ def run_ours(args):
             "peak_source": "measured in this run (hf_fp64_peak: independent DFMA chains on every SM)",
             "executed": {"achieved": EXECUTED_FLOPS_PER_ATTEMPT * probe["gpu_attempts"] / (launch_ms * 1e-3) / 1e9,
                          "flops_per_attempt": EXECUTED_FLOPS_PER_ATTEMPT,
-                         "note": "ncu FP64 instruction count per integrator step attempt (one capture of this "
-                                 "probe launch at full size) x the launch's attempts"}}
+                         "pipe_active": PROBE_FP64_PIPE,
+                         "note": "ncu FP64 instruction count per integrator step attempt (a capture of this probe "
+                                 "launch on 512 x 128 cells) x the launch's attempts; pipe_active: share of the "
+                                 "full-size launch's cycles in which the FP64 pipe is busy (ncu, 2048 x 512)"}}
     if "algorithmic" in probe:
         alg = probe["algorithmic"]
         fp64["achieved"] = alg["flops"] / (launch_ms * 1e-3) / 1e9

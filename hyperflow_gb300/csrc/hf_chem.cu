@@ -9,10 +9,10 @@
 // ChemistryBatch::advance (chemistry_batch.cpp:21-50): all-or-nothing with the
 // lowest failing index.
 //
-// The per-cell pieces (thermo, kinetics, right-hand side, Jacobian, Rodas4 step
-// attempt) are in hf_kinetics.cuh; this file holds the chemistry kernels (plain,
-// persistent, batched with its cost-ordered queue), the ErrorEst tagging kernel and
-// the allocation-free entry point.  Rate data: pre-exponential factors sit in
+// The integrators are in hf_cell.cuh (one cell per lane) and hf_group.cuh (one per group of
+// 8 lanes); this file holds the chemistry kernels (plain, persistent, batched with its
+// cost-ordered queues, small batches in groups), the ErrorEst tagging kernel and the
+// allocation-free entry point.  Rate data: pre-exponential factors sit in
 // __constant__ memory (c_A, c_A0) so they can be scaled for sensitivity checks;
 // reaction structure, temperature exponents and activation temperatures are
 // compile-time constants of the generated mechanism table, so every species index
@@ -241,13 +241,13 @@ __global__ void __launch_bounds__(64) k_chem_group(const double* __restrict__ U,
 }
 
 // Measured on the batched form (warm history): 65,536 cells of very uneven stiffness 351 ms
-// without groups, 141 with them (4,639 cells of 255 to 1,340 attempts); 512 x 128 cells with
-// 19,400 burning ones 80 ms in order of arrival, 49 with one warp of them to a
-// sub-partition; 1D detonation of 4,000 cells 149 ms (8 steps) on lanes, 58 with groups.
+// without groups, 133 with them (4,639 cells of 255 to 1,340 attempts); 512 x 128 cells with
+// 19,400 burning ones 80 ms in order of arrival, 37 to 50 with one warp of them to a
+// sub-partition; 1D detonation of 4,000 cells 149 ms (8 steps) on lanes, 40 with groups.
 //
 // Batched form: the persistent lane-refill loop of k_chem_persistent over a work
 // queue ordered most-expensive-first (order[]), starting each cell with
-// cell_begin_batched, and recording per cell the attempts taken (cost[]) and the
+// cell::begin_warm, and recording per cell the attempts taken (cost[]) and the
 // controller's proposed next step (h_hist[]) for the next call.
 template <int NS, int MINB, bool COOP>
 __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restrict__ U, int64_t cs,
@@ -565,7 +565,7 @@ cudaError_t launch_chem_batched(int ns, double* U, int64_t cs, const int64_t* id
 // Batches of the plain and persistent forms up to this many cells per SM go to
 // k_chem_group: at 64 (9,728 cells) a group for each cell costs the FP64 pipe what the lanes'
 // step chains take (29,000 pipe cycles of a sub-partition an attempt against 450,000 for 32
-// lanes).  3,000 igniting cells: 6.6 ms in groups, 16.6 on lanes.
+// lanes).  3,000 igniting cells: 5.8 ms in groups, 16.6 on lanes.
 constexpr int GROUP_CELLS_PER_SM = 64;
 template <int NS>
 static cudaError_t chem_impl(int form, double* U, int64_t cs, const int64_t* idx, int64_t count, double dt,

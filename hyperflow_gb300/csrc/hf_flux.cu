@@ -229,7 +229,8 @@ __device__ __forceinline__ bool face_flux(const Level& L, int gi, int gj, int fi
 // ---------------------------------------------------------------- plain form
 // All kernels of this path are bound by the FP64 pipe (80% active; 64 cycles of an SM
 // sub-partition per warp instruction, hf_fp64.cuh), so what they cost is their FP64
-// instruction count, measured on 1024 x 256 cells (10 species):
+// instruction count, measured on 1024 x 256 cells (10 species all present; a warp whose gas
+// lacks species leaves them out of its EOS sums, hf_device.cuh):
 //   face kernels   361 a face (1105 when limiter, comparisons and conversions were FP64
 //                  instructions and an EOS solve took two FP64 Newton steps): 0.206 ms a
 //                  direction against 0.595; of them about 230 are the two EOS solves, 65 the
@@ -237,8 +238,9 @@ __device__ __forceinline__ bool face_flux(const Level& L, int gi, int gj, int fi
 //   update         52 a cell (438 with an EOS solve to validate): 0.033 against 0.230 ms
 //   CFL            118 a cell (434): 0.070 against 0.229 ms
 // The face kernels are held to 128 registers (4 blocks an SM; 16 bytes spilled): 13.5 warps
-// in flight instead of 10.5 at 156 registers hide the integer work, 3.56 against 3.66 ms for
-// a flow of 2048 x 512 cells.
+// in flight instead of 10.5 at 156 registers hide the integer work: 3.56 against 3.66 ms for
+// a flow of 2048 x 512 cells (3.12 ms now that most of its warps sum 3 of the 10 species; 12.4
+// with all of the above as FP64 instructions).
 // Face idx of direction D of patch P into F (component stride = the patch's face count).
 template <int NS, int D, bool REC = false>
 __device__ __forceinline__ void face_one(const Level& L, const hf_patch& P, const double* __restrict__ U,
