@@ -310,7 +310,7 @@ __device__ __forceinline__ bool state_ok(const double* q, double rho) {
     bool neg = false;
     unsigned top = fp_abs_hi(rho);
 #pragma unroll
-    for (int k = 0; k < NS; ++k) neg = neg || fp_neg(q[k]);
+    for (int k = 0; k < NS; ++k) neg = neg || fp_neg_or_nan(q[k]);
 #pragma unroll
     for (int n = NS; n < NS + 3; ++n) top = max(top, fp_abs_hi(q[n]));
     return !neg && top < 0x7ff00000u && !fp_zero(rho) && __double2hiint(rho) >= 0;
@@ -422,7 +422,7 @@ __device__ __forceinline__ bool admissible_state(const double* q, double T_guess
     float lo = 0.0f, hi = 0.0f, mag = 0.0f, rho = 0.0f;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-        neg = neg || fp_neg(q[k]);
+        neg = neg || fp_neg_or_nan(q[k]);
         top = max(top, fp_abs_hi(q[k]));
         const float f = fp_to_f32(q[k]);
         rho += f;

@@ -30,9 +30,16 @@ __device__ __forceinline__ double fp_bits(unsigned long long b) {
 }
 __device__ __forceinline__ bool fp_finite(double x) { return fp_abs_hi(x) < 0x7ff00000u; }
 __device__ __forceinline__ bool fp_nan(double x) { return fp_abs_bits(x) > 0x7ff0000000000000ull; }
-// x < 0.0 and x >= 0.0 of a number (not a NaN); -0.0 is not negative
-__device__ __forceinline__ bool fp_neg(double x) { return __double2hiint(x) < 0 && !fp_zero(x); }
-__device__ __forceinline__ bool fp_ge0(double x) { return !fp_neg(x); }
+// x < 0.0 and x >= 0.0, both false for a NaN (its sign bit may be set, and the NaN of an
+// invalid operation has it set); -0.0 is not negative
+__device__ __forceinline__ bool fp_neg(double x) {
+    return __double2hiint(x) < 0 && fp_abs_bits(x) - 1 < 0x7ff0000000000000ull;
+}
+// x < 0.0 or a NaN with its sign bit set: shorter, for states that are refused for either
+__device__ __forceinline__ bool fp_neg_or_nan(double x) { return __double2hiint(x) < 0 && !fp_zero(x); }
+__device__ __forceinline__ bool fp_ge0(double x) {
+    return __double2hiint(x) >= 0 ? fp_abs_bits(x) <= 0x7ff0000000000000ull : fp_zero(x);
+}
 // x > 0.0 (false for a NaN)
 __device__ __forceinline__ bool fp_pos(double x) { return __double2hiint(x) >= 0 && !fp_zero(x) && !fp_nan(x); }
 // order of the bit patterns as integers = order of the numbers (no NaN; -0.0 < +0.0)
