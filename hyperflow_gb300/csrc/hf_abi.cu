@@ -526,7 +526,7 @@ static hf_status chem_common(hf_ctx* ctx, double* U, int64_t comp_stride, const 
     if (first_failed) *first_failed = -1;
     if (!ctx || (!U && count > 0) || count < 0 || count > INT32_MAX || (!cell_index && comp_stride < count) ||
         (!dt_cell && (!(dt > 0) || !std::isfinite(dt))) || !(rtol > 0) || !(atol > 0) ||
-        (form != HF_CHEM_PLAIN && form != HF_CHEM_PERSISTENT && form != 2))
+        (form != HF_CHEM_PLAIN && form != HF_CHEM_PERSISTENT && form != 2 && form != CHEM_GROUPS))
         return fail(ctx, HF_ERR_ARG, "chem_advance: invalid batch extent, interval or tolerances");
     if (count == 0) return HF_OK;
     const cudaStream_t s = S(stream);
@@ -948,5 +948,11 @@ hf_status record_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch*
 hf_status record_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U, double cfl,
                         double* dt, void* stream) {
     return cfl_dt(ctx, level, patch, 1, U, cfl, dt, stream, true);
+}
+hf_status record_chem_advance(hf_ctx* ctx, double* U, int64_t comp_stride, const int64_t* cell_index, int64_t count,
+                              double dt, double rtol, double atol, void* stream) {
+    int64_t first = -1;
+    return chem_common(ctx, U, comp_stride, cell_index, count, dt, nullptr, rtol, atol, CHEM_GROUPS, nullptr, &first,
+                       stream);
 }
 }  // namespace hf

@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(32) k_chem_adjoint(AdjointArgs a) {
 #pragma nv_diag_default 128
 
 // Adjoint of the react phase of a Strang step on the cells of a ghosted patch: one
-// chemistry call (plain form, the frozen accepted steps recomputed into the tape)
+// chemistry call (as recorded, its accepted steps recomputed into the tape)
 // per cell.  ubar_in = (du_out/du_in)^T ubar_out through
 //   u_in -> (y = u_k/rho, rho = sum u_k, e = E/rho - |m|^2/(2 rho^2)) -> C, Cin, et -> Rodas4
 //   steps -> y = C W/rho -> clip -> u_out_k = rho max(0, y_k), u_out_L = rho - sum u_out_k, m

@@ -582,7 +582,7 @@ static cudaError_t chem_impl(int form, double* U, int64_t cs, const int64_t* idx
                              const double* dtc, double rtol, double atol, double* trial, int* fail, DevStatus* st,
                              int sm_count, cudaStream_t s, int64_t* launches, const double* dt_dev) {
     const int bs = 64;
-    if (count <= (int64_t)sm_count * GROUP_CELLS_PER_SM) {
+    if (form == CHEM_GROUPS || count <= (int64_t)sm_count * GROUP_CELLS_PER_SM) {
         // every cell in a group of 8 lanes; both forms, so that they stay bit-identical
         const int64_t blocks = std::min<int64_t>((count + 7) / 8, (int64_t)sm_count * 4);
         k_chem_group<NS><<<(unsigned)blocks, bs, 0, s>>>(U, cs, idx, count, dt, dt_dev, dtc, rtol, atol, trial, fail, st);

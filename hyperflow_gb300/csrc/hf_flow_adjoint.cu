@@ -2,8 +2,9 @@
 // extension: the reference has no sensitivity code).
 //
 // hf_flow_record replays the loop of BlockAMR::run (HyperFlow_V3/src/BlockAMR.cpp:
-// 409-419) with the plain forms (filled ghosts + face/update kernels, one thread per
-// cell chemistry): per step flow(dt/2), react(dt), flow(dt/2), each Euler stage
+// 409-419) with the plain flux form (filled ghosts + face/update kernels) and the
+// chemistry in groups of 8 lanes, the integration that the reverse sweep recomputes bit
+// for bit, at every size: per step flow(dt/2), react(dt), flow(dt/2), each Euler stage
 // redone first order when its second-order output is inadmissible (:257-263).  It
 // records the step sizes, the first-order flags and the state every K steps.
 //
@@ -117,9 +118,8 @@ hf_status step_fwd(hf_flow_tape* t, int n, double* S0, double* const* w, double*
     if (r != HF_OK) return r;
     if (cudaMemcpyAsync(C, X, t->bytes, cudaMemcpyDeviceToDevice, s) != cudaSuccess) return HF_ERR_CUDA;
     if (t->chemistry) {
-        int64_t first = -1;
-        r = hf_chem_advance(t->ctx, C, t->P.comp_stride, t->cells, (int64_t)t->P.nx * t->P.ny, h, nullptr, t->rtol,
-                            t->atol, HF_CHEM_PLAIN, &first, s);
+        r = hf::record_chem_advance(t->ctx, C, t->P.comp_stride, t->cells, (int64_t)t->P.nx * t->P.ny, h, t->rtol,
+                                    t->atol, s);
         if (r != HF_OK) return r;
     }
     r = stage_fwd(t, C, nullptr, A2, hh, fo[2], replay, s);

@@ -66,11 +66,14 @@ void ctx_add_timing(hf_ctx* ctx, double flux_ms, double chem_ms, double other_ms
                     int64_t chem_launches, int64_t other_launches);
 
 // hf_flux_update (plain form, one patch) and hf_cfl_dt in the arithmetic of recorded runs
-// (hf_record.cuh)
+// (hf_record.cuh), and hf_chem_advance with every cell in a group at any size, as the reverse
+// sweep integrates (hf_group.cuh)
 hf_status record_flux_update(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U_in,
                              const double* U_old, double* U_out, double h, int first_order, void* stream);
 hf_status record_cfl_dt(hf_ctx* ctx, const hf_level* level, const hf_patch* patch, const double* U, double cfl,
                         double* dt, void* stream);
+hf_status record_chem_advance(hf_ctx* ctx, double* U, int64_t comp_stride, const int64_t* cell_index, int64_t count,
+                              double dt, double rtol, double atol, void* stream);
 
 // Launch wrappers (hf_flux.cu)
 cudaError_t launch_fill(int ns, const Level& L, const hf_patch* patches_host, const hf_patch* patches_dev,
@@ -159,7 +162,9 @@ cudaError_t launch_stage_adjoint(int ns, const Level& L, const hf_patch& P, cons
                                  double* inbar, DevStatus* st, cudaStream_t s, int64_t* launches);
 size_t adjoint_bytes_per_cell(int ns, int ncalls, int K, int cap);
 cudaError_t launch_chem_adjoint(int ns, const AdjointArgs& a, cudaStream_t s, int64_t* launches);
+// form: HF_CHEM_PLAIN, HF_CHEM_PERSISTENT (both in groups up to a size), or CHEM_GROUPS
 // dt_dev (nullable, plain form): read the interval from device memory instead of dt
+constexpr int CHEM_GROUPS = -1;  // every cell in a group of 8 lanes, whatever the size
 cudaError_t launch_chem(int ns, int form, double* U, int64_t comp_stride, const int64_t* cell_index,
                         int64_t count, double dt, const double* dt_cell, double rtol, double atol,
                         double* trial, int* fail, DevStatus* st, int sm_count, cudaStream_t s,

@@ -418,7 +418,8 @@ class ChemObjective(torch.autograd.Function):
 class FlowAdjoint:
     """A recorded run of Strang steps on a one-patch level and its discrete adjoint
     (hf_flow_record / hf_flow_adjoint; an extension, the reference has no sensitivity
-    code).  The run uses the plain forms with the given step sizes (or CFL steps,
+    code).  The run uses the plain flux form and the chemistry in groups of lanes, as the
+    reverse sweep integrates it, with the given step sizes (or CFL steps,
     recorded); `final` is its final state and `dts` its step sizes.
 
         fa = FlowAdjoint(ctx, level, U0, nsteps=1000, checkpoint_every=50)

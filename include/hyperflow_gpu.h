@@ -258,9 +258,9 @@ HF_EXPORT hf_status hf_chem_adjoint(hf_ctx* ctx, const double* U0, int64_t comp_
 
 /* ---- Discrete adjoint of a run of Strang steps (build-defined extension) ----
  * hf_flow_record replays nsteps steps of BlockAMR::run (BlockAMR.cpp:409-419) on a one-patch
- * level from U0 (SoA [NV][ny][nx], device) with the plain forms (ghost fill + face/update
- * kernels, one thread per cell chemistry), each stage redone first order when its output is
- * inadmissible (:257-263).  dts (host, nsteps) gives the step sizes; NULL: the CFL dt of
+ * level from U0 (SoA [NV][ny][nx], device) with the plain flux form (ghost fill + face/update
+ * kernels) and the chemistry one cell per group of 8 lanes, as the reverse sweep integrates
+ * it, each stage redone first order when its output is inadmissible (:257-263).  dts (host, nsteps) gives the step sizes; NULL: the CFL dt of
  * each step with cfl.  It records the step sizes (dts_out, host, may be NULL), the stages'
  * first-order flags and the state every checkpoint_every steps, and writes the final state
  * to U_final (device SoA, may be NULL).  No wedge boundary.  Errors as the ABI calls it
