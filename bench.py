@@ -423,7 +423,7 @@ def run_ours(args):
         m = tuning["chemistry"]["best"][0]
         tuning["stepper"] = tune.tune_stepper(ctx, level, torch.from_numpy(U0).cuda(), args.cfl, flux=flux,
                                               warm=args.warmup, steps=4,
-                                              candidates=[(m, 16), (m, 3), (m, 5), (m, 7)])
+                                              candidates=[(m, 16), (m, 17), (m, 3), (m, 5), (m, 7)])
         tuning["stepper"]["sample"] = "4 graph steps after %d warm-up steps per candidate" % args.warmup
     args.flux = flux
 

@@ -8,10 +8,12 @@
   Each candidate runs the batched chemistry three times on the same sample call (the
   chemistry input of a Strang step of the workload): the first two build the per-cell
   history (cost order, warm-started step sizes) as consecutive steps do, the third is
-  timed with CUDA events.  A candidate replaces the default only when it is more than
-  MARGIN faster on the sample: one call stands for the steps that follow, and a
+  timed with CUDA events.  The fastest is taken when it is more than MARGIN faster than
+  the setting without groups: one call stands for the steps that follow, and a
   cooperative setting whose queue stays empty on the sample can still engage, and cost,
-  in later steps.
+  in later steps.  Otherwise the setting in force stays (unless it is more than MARGIN
+  slower than the fastest): a sample that gains little from the library's own choice of
+  cells says nothing about the batches that gain 3 to 5 times from it.
 * Stepper chemistry (tune_stepper): the same settings timed over a few whole graph
   steps of the caller's stepper from one start state, each candidate from a fresh
   stepper (its history builds up over the steps as it does in a run, so a cooperative
@@ -32,21 +34,26 @@ import torch
 from . import _lib as L
 from . import solver as S
 
+# the setting without groups, which the others are measured against; the library starts at (4, 17)
 CHEM_DEFAULT = (4, 16)
-CHEM_CANDIDATES = [CHEM_DEFAULT, (4, 17), (5, 16), (6, 16), (8, 16), (4, 3), (4, 5), (4, 7)]
+CHEM_CANDIDATES = [CHEM_DEFAULT, (4, 17), (5, 17), (6, 17), (8, 17), (4, 3), (4, 5), (4, 7)]
 MARGIN = 0.03
 STEP_CANDIDATES = [CHEM_DEFAULT, (4, 17), (4, 3), (4, 5), (4, 7)]
 
 
-def pick(sweep, key, default=CHEM_DEFAULT, margin=MARGIN):
+def pick(sweep, key, default=CHEM_DEFAULT, margin=MARGIN, in_force=None):
     """The sweep entry to apply: the fastest by `key` when it is more than `margin` faster
-    than the `default` setting's entry, else the default's (the fastest when the sweep
-    has no default entry)."""
+    than the `default` setting's entry (or the sweep has no default entry); else the entry
+    of the setting `in_force`, when the sweep has one and the fastest is not more than
+    `margin` faster than it either; else the default's."""
     best = min(sweep, key=lambda r: r[key])
-    base = [r for r in sweep if (r["blocks_per_sm"], r["coop_min_bucket"]) == tuple(default)]
-    if base and best[key] >= (1.0 - margin) * base[0][key]:
-        return base[0]
-    return best
+
+    def near(setting):
+        return [r for r in sweep if (r["blocks_per_sm"], r["coop_min_bucket"]) == tuple(setting or ()) and
+                best[key] >= (1.0 - margin) * r[key]]
+
+    base = near(default)
+    return (near(in_force) or base)[0] if base else best
 
 
 def get_chem_tuning(ctx):
@@ -90,7 +97,7 @@ def tune_chemistry(ctx, X, dt, candidates=CHEM_CANDIDATES, apply=True):
             del field
     finally:
         set_chem_tuning(ctx, *before)
-    best = pick(sweep, "ms")
+    best = pick(sweep, "ms", in_force=before)
     if apply:
         set_chem_tuning(ctx, best["blocks_per_sm"], best["coop_min_bucket"])
     return {"best": (best["blocks_per_sm"], best["coop_min_bucket"]), "sweep": sweep}
@@ -122,7 +129,7 @@ def tune_stepper(ctx, level, U, cfl, flux="plain", warm=2, steps=6, candidates=S
     """U: (NV, ny, nx) state; the batched chemistry settings timed over `steps` graph steps
     (after `warm` steps) of a fresh stepper per candidate.  Returns {"best": (...),
     "sweep": [{"blocks_per_sm", "coop_min_bucket", "ms_per_step", "coop_cells"}]} and, with
-    apply, leaves the best setting in force (the default unless one beats it by MARGIN)."""
+    apply, leaves the best setting in force (as pick() chooses it)."""
     before = get_chem_tuning(ctx)
     sweep = []
     try:
@@ -146,7 +153,7 @@ def tune_stepper(ctx, level, U, cfl, flux="plain", warm=2, steps=6, candidates=S
                           "coop_cells": c1["chem_coop_cells"] - c0["chem_coop_cells"]})
     finally:
         set_chem_tuning(ctx, *before)
-    best = pick(sweep, "ms_per_step")
+    best = pick(sweep, "ms_per_step", in_force=before)
     if apply:
         set_chem_tuning(ctx, best["blocks_per_sm"], best["coop_min_bucket"])
     return {"best": (best["blocks_per_sm"], best["coop_min_bucket"]), "sweep": sweep}
