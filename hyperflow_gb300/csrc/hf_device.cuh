@@ -446,13 +446,15 @@ __device__ __forceinline__ bool admissible_state(const double* q, double T_guess
 
 // physics.cpp:40-44, one component: x y > 0 ? copysign(min(|x|, |y|), x) : 0, from the bit
 // patterns.  The product of two numbers of one sign is positive unless it underflows or
-// one is a NaN; those cases are decided by the product itself.
+// one is a NaN; those cases are decided by the product itself (as is any denormal operand,
+// whose exponent field says too little).
 __device__ __forceinline__ double minmod(double x, double y) {
     const unsigned hx = fp_abs_hi(x), hy = fp_abs_hi(y);
     const unsigned long long ax = fp_abs_bits(x), ay = fp_abs_bits(y);
     const unsigned long long lo = ax < ay ? ax : ay;
     bool pos = (__double2hiint(x) ^ __double2hiint(y)) >= 0;
-    if (hx + hy < 0x3cf00000u ? lo != 0 : max(hx, hy) >= 0x7ff00000u) pos = fp_prod_pos_lib(x, y);
+    if (hx + hy < 0x3cf00000u || min(hx, hy) < 0x00100000u ? lo != 0 : max(hx, hy) >= 0x7ff00000u)
+        pos = fp_prod_pos_lib(x, y);
     pos = pos && lo != 0;
     return __hiloint2double(pos ? (int)((unsigned)(lo >> 32) | ((unsigned)__double2hiint(x) & 0x80000000u)) : 0,
                             pos ? (int)(unsigned)lo : 0);
