@@ -279,9 +279,9 @@ __device__ __forceinline__ void secant_T(const double* w, float et, bool& low, f
 }
 
 // The same for a specific energy e (J/kg) and weights z_k = Y_k / W_k, from a warm guess:
-// FP32 Newton with both ranges' coefficients, then solve_T_any (two FP64 iterations).  Less
-// code than the form above, which is what the chemistry kernel, bound by instruction
-// fetch, needs.
+// FP32 Newton with both ranges' coefficients, then solve_T_any (two FP64 iterations).  Kept for
+// the arithmetic of recorded runs (hf_record.cuh) and the derivatives of an objective
+// (hf_adjoint.cu).
 template <int NS, int RG>
 __device__ __forceinline__ void mix_coef_f(const double* z, float* m) {
 #pragma unroll
@@ -342,11 +342,38 @@ __device__ __forceinline__ bool state_ok(const double* q, double rho) {
 // measured fields' states, against 80 bits) of p, a and T: 1.1 to 1.6, 0.9 to 1.1 and 0.9 to
 // 1.4 e-16; with the operators, mass fractions and two FP64 Newton steps 1.4 to 2.5, 0.9 to 1.4
 // and 1.2 to 1.3.
-// Species whose partial density is below 2^-110 of the largest add less than 2^-98 of the
-// largest term of any sum formed here (the coefficients' ratios stay below 2^12): no sum
-// changes by a bit unless its terms cancel to 2^-45, so a warp in which all lanes agree on
-// it leaves such species out.  In unburnt gas that is 7 of 10, and a solve takes 58 FP64
-// instructions instead of 114.
+// Species whose partial density is below 2^-110 of the largest are left out of the sums by a
+// warp in which all lanes agree on it.  Together they change the density, the heat capacity,
+// sum q_k / W_k and, through the energy, T by less than 2^-94 of each (trace_bound): far below a
+// rounding.  (A single coefficient of the mixture may lose all it has: H and AR have zeros in
+// four.)  In unburnt gas that is 7 of 10, and a solve takes 58 FP64 instructions instead of 114.
+constexpr double TRACE_RATIO = 65536.0;  // 2^16: times 2^-110
+constexpr double abs_of(double x) { return x < 0 ? -x : x; }
+constexpr bool trace_bound() {
+    const ECoef e = make_ecoef_mass();
+    const InvW w = make_rinvw();
+    double w_lo = 1e300, w_hi = 0.0;
+    for (int k = 0; k < NS_MAX; ++k) {
+        w_lo = w.v[k] < w_lo ? w.v[k] : w_lo;
+        w_hi = w.v[k] > w_hi ? w.v[k] : w_hi;
+    }
+    if (!(NS_MAX * w_hi < TRACE_RATIO * w_lo)) return false;
+    for (double T = T_LO; T <= T_HI; T += 25.0) {
+        double cv_lo = 1e300, cv_hi = 0.0, e_hi = 0.0;
+        for (int k = 0; k < NS_MAX; ++k) {
+            const double(&c)[6] = e.c[T <= TMID ? 0 : 1][k];
+            const double cv = (((5.0 * c[4] * T + 4.0 * c[3]) * T + 3.0 * c[2]) * T + 2.0 * c[1]) * T + c[0];
+            const double en = abs_of(ecoef_at(c, T));
+            cv_lo = cv < cv_lo ? cv : cv_lo;
+            cv_hi = cv > cv_hi ? cv : cv_hi;
+            e_hi = en > e_hi ? en : e_hi;
+        }
+        // of the energy against cv T of the largest species: what it moves T by
+        if (!(cv_lo > 0.0 && NS_MAX * cv_hi < TRACE_RATIO * cv_lo && NS_MAX * e_hi < TRACE_RATIO * cv_lo * T)) return false;
+    }
+    return true;
+}
+static_assert(trace_bound(), "a trace species can matter: the cut of live_species is too high for this mechanism");
 template <int NS>
 __device__ __forceinline__ unsigned live_species(const double* q) {
     unsigned top = 0, live = 0;
