@@ -26,35 +26,30 @@ namespace hf {
 
 cudaError_t adjoint_set_rate_scale(const double* scale) { return upload_rate_constants(scale); }
 
-// cp/R and d(cp/R)/dT of every species
+// cp/R of every species
 template <int NS>
-__device__ __forceinline__ void species_cp(double T, double* cpR, double* dcpR) {
+__device__ __forceinline__ void species_cp(double T, double* cpR) {
     const int rg = T <= TMID ? 0 : 1;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         const double* a = D_NASA.c[rg][k];
         cpR[k] = fma(T, fma(T, fma(T, fma(T, a[4], a[3]), a[2]), a[1]), a[0]);
-        dcpR[k] = fma(T, fma(T, fma(T, 4.0 * a[4], 3.0 * a[3]), 2.0 * a[2]), a[1]);
     }
 }
 
 // Constant-(rho, e) temperature derivatives at y (R units: e_k/R = T (h_k/RT - 1)/W_k,
 // cv_k/R = (cp_k/R - 1)/W_k):  dT/dy_j = -(e_j - e_L)/cv.
 template <int NS>
-__device__ __forceinline__ void temp_grad(const KinCtx<NS>& kc, const double* cpR, const double* y, double* dTdy,
-                                          double* cvk, double& cv, double& ETT, const double* dcpR) {
+__device__ __forceinline__ void temp_grad(const KinCtx<NS>& kc, const double* cpR, const double* y, double* dTdy) {
     constexpr int N = NS - 1, L = NS - 1;
     double YL = 1.0;
 #pragma unroll
     for (int k = 0; k < N; ++k) YL -= y[k];
-    cv = 0.0;
-    ETT = 0.0;
+    double cv = 0.0;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-        cvk[k] = (cpR[k] - 1.0) * INVW.v[k];
         const double Yk = k < N ? y[k] : YL;
-        cv = fma(Yk, cvk[k], cv);
-        if (dcpR) ETT = fma(Yk, dcpR[k] * INVW.v[k], ETT);
+        cv = fma(Yk, (cpR[k] - 1.0) * INVW.v[k], cv);
     }
     const double eL = kc.T * (kc.hRT[L] - 1.0) * INVW.v[L];
 #pragma unroll
@@ -78,9 +73,9 @@ __device__ bool state_grads(const double* u, double* dT, double* dp, double& T) 
     if (!solve_T_iter<NS>(z, e, T, m)) return false;
     KinCtx<NS> kc;
     kin_setup<NS, false>(T, C, kc);
-    double cpR[NS], dcpR[NS], cvk[NS], cv, ETT;
-    species_cp<NS>(T, cpR, dcpR);
-    temp_grad<NS>(kc, cpR, y, dT, cvk, cv, ETT, nullptr);
+    double cpR[NS];
+    species_cp<NS>(T, cpR);
+    temp_grad<NS>(kc, cpR, y, dT);
     double zs = 0.0;
 #pragma unroll
     for (int k = 0; k < NS; ++k) zs += z[k];
@@ -457,7 +452,7 @@ __global__ void __launch_bounds__(32) k_chem_call_adjoint(hf_patch P, const doub
     const int r = run_call<NS>(uc, dt, rtol, atol, tape + li, chunk, nrec, cap, clip, yend, live, &sh->f);
     bool ok = live && r == CELL_DONE && nrec <= cap;
     const Interval<NS> v = interval<NS>(u);
-    const double mx = u[NS], my = u[NS + 1], E = u[NS + 2], ir = v.ir;
+    const double mx = u[NS], my = u[NS + 1], ir = v.ir;
     // output side: u_out_k = rho Y'_k (k < N), u_out_L = rho (1 - sum Y'_k)
     double lam = 0.0, lamN2 = 0.0, rhob = ub[N];
 #pragma unroll
@@ -505,7 +500,6 @@ __global__ void __launch_bounds__(32) k_chem_call_adjoint(hf_patch P, const doub
 #pragma unroll
     for (int n = 0; n < NV; ++n)
         if ((n & 7) == t) ubar_in[g + n * P.comp_stride] = ok ? out[n] : 0.0;
-    (void)E;
 }
 
 }  // namespace

@@ -608,7 +608,6 @@ static __device__ __noinline__ void swap_rows8(unsigned swaps, double* b) {
                 b[i] = t;
             }
 }
-template <int STR>
 __device__ __forceinline__ void solve8(const double* Lu, unsigned swaps, double* b) {
     if (swaps) {
         double t[NQ];
@@ -621,12 +620,12 @@ __device__ __forceinline__ void solve8(const double* Lu, unsigned swaps, double*
 #pragma unroll
     for (int i = 1; i < NQ; ++i)
 #pragma unroll
-        for (int j = 0; j < i; ++j) b[i] = fma(-Lu[(i * NQ + j) * STR], b[j], b[i]);
+        for (int j = 0; j < i; ++j) b[i] = fma(-Lu[(i * NQ + j)], b[j], b[i]);
 #pragma unroll
     for (int i = NQ - 1; i >= 0; --i) {
 #pragma unroll
-        for (int j = i + 1; j < NQ; ++j) b[i] = fma(-Lu[(i * NQ + j) * STR], b[j], b[i]);
-        b[i] *= Lu[(i * NQ + i) * STR];
+        for (int j = i + 1; j < NQ; ++j) b[i] = fma(-Lu[(i * NQ + j)], b[j], b[i]);
+        b[i] *= Lu[(i * NQ + i)];
     }
 }
 
@@ -641,7 +640,7 @@ enum : int { LU_OK = 0, LU_RHS_FAILED, LU_SINGULAR, LU_SCREENED, LU_COLD };
 // 1e-5, the interval is taken as one second-order Taylor step y1 = y0 + dt f0 + dt^2/2 J f0:
 // for the linearised system its remainder sum_{k>=3} dt^k/k! J^(k-1) f0 is bounded by the
 // last expression, i.e. below 1e-5 tolerance units.
-template <int NS, bool SCREEN, int STR>
+template <int NS, bool SCREEN>
 __device__ __noinline__ int jac_lu(Cell<NS>& c, const double* Cm, double* f0, double* Lu, unsigned& swaps, double inv,
                                    double rtol, double atol) {
     double C[NQ], w[NQ], A[NQ * NQ], Tn[NQ], Dn[NQ], h[NQ], Csum, cv, T = c.T;
@@ -711,7 +710,7 @@ __device__ __noinline__ int jac_lu(Cell<NS>& c, const double* Cm, double* f0, do
     for (int i = 0; i < NQ; ++i) A[i * NQ + i] += inv;
     if (!lu8(A, swaps)) return LU_SINGULAR;
 #pragma unroll
-    for (int i = 0; i < NQ * NQ; ++i) Lu[i * STR] = A[i];
+    for (int i = 0; i < NQ * NQ; ++i) Lu[i] = A[i];
     return LU_OK;
 }
 
@@ -827,9 +826,9 @@ __device__ __forceinline__ int begin_warm(Cell<NS>& c, const double* u, double d
     return CELL_CONTINUE;
 }
 
-// One step attempt (the body of the KPP accept loop).  Lu: 64 doubles of scratch at stride
-// STR; screened is set when a frozen cell was finished by the screen.
-template <int NS, bool SCREEN, int STR>
+// One step attempt (the body of the KPP accept loop).  Lu: 64 doubles of scratch;
+// screened is set when a frozen cell was finished by the screen.
+template <int NS, bool SCREEN>
 __device__ __forceinline__ int attempt(Cell<NS>& c, double rtol, double atol, double* Lu, bool* screened = nullptr) {
     double C0[NQ], K[6][NQ], Ys[NQ];
     unsigned swaps = 0;
@@ -843,7 +842,7 @@ __device__ __forceinline__ int attempt(Cell<NS>& c, double rtol, double atol, do
     const double ih = fp_pos(h) ? fp_rcp(h) : 0.0;
 #pragma unroll
     for (int i = 0; i < NQ; ++i) Ys[i] = C0[i] = c.rho * c.y[i] * INVW.v[i];
-    const int r = jac_lu<NS, SCREEN, STR>(c, C0, K[0], Lu, swaps, ih * (1.0 / RGAMMA), rtol, atol);
+    const int r = jac_lu<NS, SCREEN>(c, C0, K[0], Lu, swaps, ih * (1.0 / RGAMMA), rtol, atol);
     if (r == LU_RHS_FAILED) return CELL_FAIL;
     if (SCREEN) {
         if (r == LU_SCREENED) {
@@ -861,7 +860,7 @@ __device__ __forceinline__ int attempt(Cell<NS>& c, double rtol, double atol, do
         double b[NQ];
 #pragma unroll
         for (int i = 0; i < NQ; ++i) b[i] = K[0][i];
-        solve8<STR>(Lu, swaps, b);
+        solve8(Lu, swaps, b);
 #pragma unroll
         for (int i = 0; i < NQ; ++i) K[0][i] = b[i];
     }
@@ -892,7 +891,7 @@ __device__ __forceinline__ int attempt(Cell<NS>& c, double rtol, double atol, do
         if (!ok) break;
 #pragma unroll
         for (int i = 0; i < NQ; ++i) b[i] = fma(ih, b[i], f[i]);
-        solve8<STR>(Lu, swaps, b);
+        solve8(Lu, swaps, b);
 #pragma unroll
         for (int i = 0; i < NQ; ++i) K[s][i] = b[i];
     }

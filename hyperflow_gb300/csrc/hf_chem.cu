@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(64) k_chem_plain(const double* __restrict__ U,
     double Lu[cell::NQ * cell::NQ];
     c.attempts = 0;
     int r = cell::begin<NS>(c, u, dt_cell ? dt_cell[i] : dt, rtol, atol);
-    while (r == CELL_CONTINUE) r = cell::attempt<NS, false, 1>(c, rtol, atol, Lu);
+    while (r == CELL_CONTINUE) r = cell::attempt<NS, false>(c, rtol, atol, Lu);
     atomicAdd(&st->steps, (unsigned long long)c.attempts);
     if (r == CELL_DONE && cell::finish<NS>(c, u)) {
 #pragma unroll
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(64) k_chem_persistent(const double* __restrict
             continue;
         }
         if (active) {
-            const int r = cell::attempt<NS, false, 1>(c, rtol, atol, Lu);
+            const int r = cell::attempt<NS, false>(c, rtol, atol, Lu);
             if (r != CELL_CONTINUE) {
                 my_attempts += c.attempts;
                 double u[NS + 3];
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(64, MINB) k_chem_batched(const double* __restr
             }
             if (active) {
                 bool screened = false;
-                const int r = cell::attempt<NS, true, 1>(c, rtol, atol, Lu, &screened);
+                const int r = cell::attempt<NS, true>(c, rtol, atol, Lu, &screened);
                 if (r != CELL_CONTINUE) {
                     my_attempts += c.attempts;
                     double u[NS + 3];

@@ -90,7 +90,7 @@ constexpr InvW make_rinvw() {
     return w;
 }
 __device__ constexpr InvW RINVW = make_rinvw();
-// e_k(T) W_k / R at the temperatures that bracket the solve, and e_k(T)
+// e_k(T) at the temperatures that bracket the solve
 constexpr double T_LO = 250.0, T_HI = 5000.0;
 struct EAt { double lo[NS_MAX], mid[NS_MAX], hi[NS_MAX]; };
 constexpr double ecoef_at(const double (&c)[6], double T) {
@@ -105,7 +105,6 @@ constexpr EAt make_eat(const ECoef& e) {
     }
     return a;
 }
-__device__ constexpr EAt D_EAT = make_eat(make_ecoef());
 __device__ constexpr EAt D_EAT_MASS = make_eat(make_ecoef_mass());
 
 // Mixture polynomial of one NASA range: e(T)/R = sum_j m[j] T^(j+1) + m[5], with
@@ -263,15 +262,15 @@ __device__ __forceinline__ bool newton_T(const double* m, double et, bool low, f
     }
     return false;
 }
-template <int NS, bool MASS>
+template <int NS>
 __device__ __forceinline__ void secant_T(const double* w, float et, bool& low, float& t) {
     float lo = 0.0f, mid = 0.0f, hi = 0.0f;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         const float f = fp_to_f32(w[k]);
-        lo = fmaf(f, (float)(MASS ? D_EAT_MASS.lo[k] : D_EAT.lo[k]), lo);
-        mid = fmaf(f, (float)(MASS ? D_EAT_MASS.mid[k] : D_EAT.mid[k]), mid);
-        hi = fmaf(f, (float)(MASS ? D_EAT_MASS.hi[k] : D_EAT.hi[k]), hi);
+        lo = fmaf(f, (float)D_EAT_MASS.lo[k], lo);
+        mid = fmaf(f, (float)D_EAT_MASS.mid[k], mid);
+        hi = fmaf(f, (float)D_EAT_MASS.hi[k], hi);
     }
     low = et <= mid;
     t = low ? (float)T_LO + (et - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
@@ -413,7 +412,7 @@ __device__ __forceinline__ bool properties(const double* q, Props& s, double T_g
     {
         float t;
         bool low;
-        secant_T<NS, true>(q, fp_to_f32(et), low, t);
+        secant_T<NS>(q, fp_to_f32(et), low, t);
         if (low) mix_live<NS, 0>(q, live, m);
         else mix_live<NS, 1>(q, live, m);
         if (!newton_T(m, et, low, t, T, cv)) {
@@ -447,7 +446,7 @@ template <int NS>
 __device__ __forceinline__ double estimate_T(const double* q, double et) {
     float t;
     bool low;
-    secant_T<NS, true>(q, (float)RU * fp_to_f32(et), low, t);
+    secant_T<NS>(q, (float)RU * fp_to_f32(et), low, t);
     return t > 50.0f && t < 9000.0f ? fp_from_f32(t) : 1000.0;
 }
 
