@@ -26,12 +26,14 @@ def text():
     # k up to 21 bits: k * STEP_HI is exact; LN2_HI likewise for exponents of 11 bits
     hi, lo = split(step, 32)
     l_hi, l_lo = split(LN2, 42)
+    r = step * Decimal("0.51")  # bound of the reduced argument
+    c2 = float(Decimal("0.5") + r * r / 24)
     out = ["// Written by gen_exptab.py: tables of the short exponential and logarithm (hf_cell.cuh).",
            "#pragma once", "namespace hf {", "namespace et {",
            "constexpr double STEP_HI = %s;  // ln2 / %d = HI + LO" % (hi.hex(), NE),
            "constexpr double STEP_LO = %s;" % lo.hex(),
            "constexpr float INV_STEP = %.9ef;  // %d / ln2" % (float(1 / step), NE),
-           "constexpr double C2 = %s;  // of r^2 in exp(r)" % (0.5).hex(),
+           "constexpr double C2 = %s;  // 1/2 + R^2/24, R = 0.51 ln2 / %d" % (c2.hex(), NE),
            "constexpr double LN2_HI = %s;" % l_hi.hex(),
            "constexpr double LN2_LO = %s;" % l_lo.hex()]
     for name, vals in (("EXP", exp_tab), ("LOG_IF", [float(1 / f) for f in F]), ("LOG_F", [float(f.ln()) for f in F])):

@@ -34,12 +34,10 @@ namespace cell {
 
 constexpr int NQ = 8;  // reacting species: H2, O2, H2O, H, O, OH, HO2, H2O2
 
-// exp(x), |x| < 340: x = k ln2/2048 + r, k from the FP32 product of x cut to FP32, so |r| <=
-// 0.64 ln2/2048 = 2.17e-4; 2^(k/2048) from a table, exp(r) - 1 = r + r^2/2 + r^3 (1/6 + r/24),
-// the bracket in FP32 (r^3 is below 1.1e-11, so its rounding is below 4e-19 and the next term
-// below 4e-21).  6 FP64 instructions; table and result round to half a unit each: within 1.01
-// ulp (1.06 without the r^4 term).  After P. T. P. Tang's table-driven exponential (ACM TOMS 15
-// (1989) 144-157).  Other arguments: the library function.
+// exp(x), |x| < 340: x = k ln2/2048 + r, k from the FP32 product (|r| <= 0.51 ln2/2048),
+// 2^(k/2048) from a table, exp(r) - 1 = r + C2 r^2 + r^3/6 with C2 the economised 1/2.
+// 6 FP64 instructions, within 1.5 ulp; after P. T. P. Tang's table-driven exponential (ACM
+// TOMS 15 (1989) 144-157).  Other arguments: the library function.
 __device__ __forceinline__ bool small_arg(double x) { return fp_abs_hi(x) < 0x40754000u; }
 __device__ __forceinline__ double reduce(double x, int& k) {
     k = __float2int_rn(fp_to_f32(x) * et::INV_STEP);
@@ -50,12 +48,11 @@ __device__ __forceinline__ double fexp(double x) {
     if (!small_arg(x)) return fm_exp_lib(x);
     int k;
     const double r = reduce(x, k);
-    const double c = fp_from_f32(fmaf(fp_to_f32(r), 1.0f / 24.0f, 1.0f / 6.0f));
-    const double p = fma(r * r, fma(r, c, et::C2), r);
+    const double p = fma(r * r, fma(r, 1.0 / 6.0, et::C2), r);
     const double t = et::EXP[k & 2047];
     return fm_scale(fma(t, p, t), k >> 11);
 }
-// exp(x) and exp(-x): 10 FP64 instructions
+// exp(x) and exp(-x): 9 FP64 instructions
 __device__ __forceinline__ void fexp_pair(double x, double& ep, double& em) {
     if (!small_arg(x)) {
         ep = fm_exp_lib(x);
@@ -64,16 +61,15 @@ __device__ __forceinline__ void fexp_pair(double x, double& ep, double& em) {
     }
     int k;
     const double r = reduce(x, k);
-    const double r2 = r * r, o = fma(r, r2 * (1.0 / 6.0), r), c = fma(r2, 1.0 / 24.0, et::C2);
+    const double r2 = r * r, o = fma(r, r2 * (1.0 / 6.0), r);
     const double tp = et::EXP[k & 2047], tm = et::EXP[-k & 2047];
-    ep = fm_scale(fma(tp, fma(c, r2, o), tp), k >> 11);
-    em = fm_scale(fma(tm, fma(c, r2, -o), tm), -k >> 11);
+    ep = fm_scale(fma(tp, fma(et::C2, r2, o), tp), k >> 11);
+    em = fm_scale(fma(tm, fma(et::C2, r2, -o), tm), -k >> 11);
 }
 // log(x) of a positive normal number: x = 2^m y, F = 1 + (j + 1/2)/256, u = (y - F)/F,
-// |u| <= 1/513; log1p(u) = u - u^2/2 + u^3 (1/3 - u/4 + u^2/5 - u^3/6), of the bracket all but
-// the 1/3 in FP32 (its rounding is below 1e-18 of log1p; with the 1/3 in FP32 too it was 2e-16,
-// two units of the last place near x = 1).  9 FP64 instructions; after Tang, ACM TOMS 16 (1990)
-// 378-400.
+// |u| <= 1/513; log1p(u) = u - u^2/2 + u^3 (1/3 - u/4 + u^2/5), the bracket in FP32 (its
+// rounding is below 2e-16 of the result's terms).  8 FP64 instructions; after Tang, ACM
+// TOMS 16 (1990) 378-400.
 __device__ __forceinline__ double flog(double x) {
     const int hi = __double2hiint(x);
     if ((unsigned)hi - 0x00200000u >= 0x7fc00000u) return fm_log_lib(x);
@@ -83,7 +79,7 @@ __device__ __forceinline__ double flog(double x) {
     const double F = __hiloint2double((yh & (int)0xfffff000) | 0x800, 0);
     const double u = (y - F) * et::LOG_IF[j];
     const float f = fp_to_f32(u);
-    const double q = 1.0 / 3.0 + fp_from_f32(f * fmaf(f, fmaf(f, -1.0f / 6.0f, 0.2f), -0.25f));
+    const double q = fp_from_f32(fmaf(f, fmaf(f, 0.2f, -0.25f), 1.0f / 3.0f));
     const double l = fma(u * u, fma(u, q, -0.5), u);
     const double m = fp_from_f32((float)((hi >> 20) - 1023));
     return fma(m, et::LN2_HI, et::LOG_F[j]) + fma(m, et::LN2_LO, l);
