@@ -106,6 +106,15 @@ constexpr EAt make_eat(const ECoef& e) {
     return a;
 }
 __device__ constexpr EAt D_EAT_MASS = make_eat(make_ecoef_mass());
+// the same over R, for the chemistry, whose energies are rho e / R
+constexpr ECoef make_ecoef_mass_R() {
+    ECoef e = make_ecoef();
+    for (int r = 0; r < 2; ++r)
+        for (int k = 0; k < NS_MAX; ++k)
+            for (int j = 0; j < 6; ++j) e.c[r][k][j] /= MW[k];
+    return e;
+}
+__device__ constexpr EAt D_EAT_R = make_eat(make_ecoef_mass_R());
 
 // Mixture polynomial of one NASA range: e(T)/R = sum_j m[j] T^(j+1) + m[5], with
 // m[j] = sum_k w_k c_kj for weights w_k: moles (z_k = Y_k / W_k, or concentrations) or,
@@ -262,15 +271,15 @@ __device__ __forceinline__ bool newton_T(const double* m, double et, bool low, f
     }
     return false;
 }
-template <int NS>
+template <int NS, bool PER_R = false>
 __device__ __forceinline__ void secant_T(const double* w, float et, bool& low, float& t) {
     float lo = 0.0f, mid = 0.0f, hi = 0.0f;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         const float f = fp_to_f32(w[k]);
-        lo = fmaf(f, (float)D_EAT_MASS.lo[k], lo);
-        mid = fmaf(f, (float)D_EAT_MASS.mid[k], mid);
-        hi = fmaf(f, (float)D_EAT_MASS.hi[k], hi);
+        lo = fmaf(f, (float)(PER_R ? D_EAT_R.lo[k] : D_EAT_MASS.lo[k]), lo);
+        mid = fmaf(f, (float)(PER_R ? D_EAT_R.mid[k] : D_EAT_MASS.mid[k]), mid);
+        hi = fmaf(f, (float)(PER_R ? D_EAT_R.hi[k] : D_EAT_MASS.hi[k]), hi);
     }
     low = et <= mid;
     t = low ? (float)T_LO + (et - lo) * ((float)(TMID - T_LO) * fp_rcp_seed(mid - lo))
@@ -431,7 +440,7 @@ __device__ __forceinline__ bool properties(const double* q, Props& s, double T_g
     s.p = T * zs;
     // a^2 = (1 + zs / cv) p / rho: zs / cv, rounded twice, is 0.2 to 0.7 of the sum
     const double P = s.p * ir;
-    s.a = fp_sqrt(fma(P, zs * fp_rcp(cv), P));
+    s.a = fp_sqrt_near(fma(P, zs * fp_rcp(cv), P));
     return fp_pos(s.T) && fp_pos(s.p) && fp_pos(s.a) && fp_finite(s.a);
 }
 template <int NS>
@@ -446,7 +455,7 @@ template <int NS>
 __device__ __forceinline__ double estimate_T(const double* q, double et) {
     float t;
     bool low;
-    secant_T<NS>(q, (float)RU * fp_to_f32(et), low, t);
+    secant_T<NS, true>(q, fp_to_f32(et), low, t);
     return t > 50.0f && t < 9000.0f ? fp_from_f32(t) : 1000.0;
 }
 

@@ -4,8 +4,8 @@
 // lanes and independent chains; so does every FP64 <-> FP32 or integer conversion (56 to
 // 64 cycles).  An integer or FP32 instruction takes 1 or 2.  So comparisons, signs,
 // minima and conversions are done on the bit patterns here, and reciprocals, quotients
-// and square roots start from an FP32 seed and take 3, 5 and 5 FP64 instructions (the
-// operators: about 5.5, 8.8 and 9.5 by the same measurement).
+// and square roots start from an FP32 seed and take 3, 5 and 4 or 5 FP64 instructions
+// (the operators: about 5.5, 8.8 and 9.5 by the same measurement).
 //
 // Reciprocal: Householder's iteration of third order, r = r0 (1 + e + e^2), e = 1 - x r0,
 // from an FP32 seed with |e| <= 2^-21: the remainder e^3 is below 2^-63.  Square root: the
@@ -114,9 +114,18 @@ __device__ __forceinline__ double fp_div(double a, double b) {
     const double q = a * r;
     return fma(fma(-b, q, a), r, q);
 }
-// sqrt(x): h = x y rounds, and its own remainder x - h^2 (exact) corrects it, so the result is off
-// by half a unit and 2^-40 of one
+// sqrt(x) within 1 ulp (norms and step sizes)
 __device__ __forceinline__ double fp_sqrt(double x) {
+    if (__double2hiint(x) < 0 || !fp_seedable(x)) return fp_sqrt_lib(x);
+    const double y = fp_from_f32(fp_rsqrt_seed(fp_to_f32(x)));
+    const double t = x * y;
+    const double e = fma(-t, y, 1.0);
+    const float f = fp_to_f32(e);
+    return fma(t, fma(0.5, e, fp_from_f32(0.375f * f * f)), t);
+}
+// sqrt(x): h = x y rounds, and its own remainder x - h^2 (exact) corrects it, so the result is off
+// by half a unit and 2^-10 of one; one instruction more
+__device__ __forceinline__ double fp_sqrt_near(double x) {
     if (__double2hiint(x) < 0 || !fp_seedable(x)) return fp_sqrt_lib(x);
     const double y = fp_from_f32(fp_rsqrt_seed(fp_to_f32(x)));
     const double h = x * y, t = fma(-h, h, x) * y;  // sqrt(x) = h + t (1/2 + 3/8 e + ...), e = t / sqrt(x)
