@@ -26,7 +26,7 @@ def text():
     # k up to 21 bits: k * STEP_HI is exact; LN2_HI likewise for exponents of 11 bits
     hi, lo = split(step, 32)
     l_hi, l_lo = split(LN2, 42)
-    r = step * Decimal("0.51")  # bound of the reduced argument
+    r = step * Decimal("0.51")  # C2 fits this far; the reduced argument reaches 0.65 of a step
     c2 = float(Decimal("0.5") + r * r / 24)
     out = ["// Written by gen_exptab.py: tables of the short exponential and logarithm (hf_cell.cuh).",
            "#pragma once", "namespace hf {", "namespace et {",

@@ -135,11 +135,15 @@ HF_EXPORT void hf_get_chem_tuning(int32_t* blocks_per_sm, int32_t* coop_min_buck
  * of three timed launches after a warm-up.  Measurement utility; no reference counterpart. */
 HF_EXPORT hf_status hf_fp64_peak(hf_ctx* ctx, double* gflops, void* stream);
 
-/* The chemistry kernels' table-driven exponential and logarithm on n device values:
- * exp_out = exp(x); pair_pos, pair_neg = exp(x), exp(-x) from the paired form;
- * log_out = log(x).  Check utility (within a few ulp of the correctly rounded values);
+/* The table-driven exponential and logarithm of the tagging and adjoint objective kernels on
+ * n device values: exp_out = exp(x); pair_pos, pair_neg = exp(x), exp(-x) from the paired
+ * form; log_out = log(x).  Check utility (within a few ulp of the correctly rounded values);
  * no reference counterpart. */
 HF_EXPORT hf_status hf_fastmath_eval(const double* x, int64_t n, double* exp_out, double* pair_pos, double* pair_neg,
+                                     double* log_out, void* stream);
+/* The same of the shorter forms that the chemistry integrators evaluate (exp within 1.35
+ * units in the last place; log within 1.5 units and 2.7e-16). */
+HF_EXPORT hf_status hf_cellmath_eval(const double* x, int64_t n, double* exp_out, double* pair_pos, double* pair_neg,
                                      double* log_out, void* stream);
 
 /* ---- EOS / flux primitives on batches (physics.cpp:4-48) ---- */
