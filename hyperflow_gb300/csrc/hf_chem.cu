@@ -384,10 +384,10 @@ void chem_tuning(int* minb, int* coop_min) {
     *coop_min = g_tune_coop.load();
 }
 
-// Work-queue order: counting sort of cells by bucket = floor(log2(cost + 1)) (16
-// buckets), most expensive bucket first.  Cells of one bucket keep no particular
-// order; each cell's result does not depend on its position.
-// With SUB sub-buckets to a factor of two the cells of a warp have about the same cost.
+// Work-queue order: counting sort of the cells by cost bin, most expensive bin first: SUB bins
+// to a factor of two of cost + 1, 128 in all, so that the cells of a warp have about the same
+// cost.  Cells of one bin keep no particular order; a cell's result does not depend on its place
+// in the queue, only (to rounding) on whether its bin goes to groups.
 constexpr int NBUCKET = 16, SUB = 8, NBIN = NBUCKET * SUB;
 constexpr int COSTLY_BUCKET = 4;  // at least 15 attempts
 static_assert(NBIN + 2 <= CHEM_BINS, "bins");

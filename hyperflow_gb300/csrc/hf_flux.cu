@@ -237,10 +237,12 @@ __device__ __forceinline__ bool face_flux(const Level& L, int gi, int gj, int fi
 //                  reconstruction
 //   update         52 a cell (438 with an EOS solve to validate): 0.033 against 0.230 ms
 //   CFL            118 a cell (434): 0.070 against 0.229 ms
-// The face kernels are held to 128 registers (4 blocks an SM; 16 bytes spilled): 13.5 warps
-// in flight instead of 10.5 at 156 registers hide the integer work: 3.56 against 3.66 ms for
-// a flow of 2048 x 512 cells (3.12 ms now that most of its warps sum 3 of the 10 species; 12.4
-// with all of the above as FP64 instructions).
+// The face kernels are held to 128 registers (4 blocks an SM): 13.5 warps in flight instead of
+// 10.5 at 156 registers hide the integer work: 3.56 against 3.66 ms for a flow of 2048 x 512
+// cells (3.10 ms now that most of its warps sum 3 of the 10 species; 12.4 with all of the above
+// as FP64 instructions).  The one-patch kernels spill nothing or 4 bytes under that bound; those
+// over all patches of a level, which carry the patch's fields too, 92 to 140 bytes, and were
+// not measured without it.
 // Face idx of direction D of patch P into F (component stride = the patch's face count).
 template <int NS, int D, bool REC = false>
 __device__ __forceinline__ void face_one(const Level& L, const hf_patch& P, const double* __restrict__ U,
@@ -456,8 +458,12 @@ cudaError_t launch_flux_plain(int ns, const Level& L, const hf_patch& P, int, co
 // thread updates, validates and (optionally) Heun-combines one cell.
 // A 32 x 7 tile has (TX+1) TY + TX (TY+1) = 487 faces, which 8 warps take in two
 // passes (a 32 x 8 tile has 552: a third, nearly empty pass that the other warps wait
-// for at the barrier); the first TX x TY threads then update one cell each.  Nine
-// warps would cap registers at 168 (three warps on one scheduler) and spill.
+// for at the barrier); the first TX x TY threads then update one cell each.  128
+// registers (120 bytes spilled with 10 species, 40 with 9) and 92 KB of shared memory: two
+// CTAs an SM, 15.4 warps in flight, FP64 pipe 77% active (512 x 128 cells).  8.7% of the
+// faces are evaluated in two tiles and a tile's last warp pass is a quarter full, so a stage
+// takes 789 FP64 instructions a cell there where the plain kernels take 669; 1.64 against 1.31
+// ms on 2048 x 512 cells.
 constexpr int TX = 32, TY = 7, HX = TX + 4, HY = TY + 4, NTHR = 256;
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }

@@ -13,11 +13,13 @@
 // its gradient is the tangent, along (beta_r, d lnT = tau . beta_r), of reaction r's own
 // partial derivatives, plus the curvature of T(C, Cin, et).
 //
-// What bounds it: the step chain of a cell (the FP64 latency of one warp).  The stages'
-// partial derivatives are kept in shared memory from the forward recomputation (8 KB a
-// cell), so the transposed products cost a sixth of an evaluation each: about 3,000 FP64
-// instructions a step for four cells, against 130,000 FP64 instruction times for 32 cells on
-// one lane each.
+// What bounds it: the step chain of a cell, about 250 us a reverse step with the forward attempt
+// it follows (73 us).  The stages' partial derivatives are kept in shared memory from the forward
+// recomputation (8 KB a cell), so the transposed products cost a sixth of an evaluation each:
+// about 3,000 FP64 instructions a step for four cells, against 130,000 FP64 instruction times
+// for 32 cells on one lane each.  Those 3,000 hold the pipe for 93 us; what the rest of the
+// step waits for (table and weight loads ahead of dependent shared loads, the tape's strided
+// loads, shuffles) was not separated.
 #pragma once
 #include "hf_group.cuh"
 

@@ -7,8 +7,8 @@
 // Two ways through a step:
 //  * graph path (CFL dt, either chemistry form): the whole Strang step - CFL
 //    reduction, dt on the device, four Euler stages (fused kernel, or ghost fill + face
-//    + update kernels of the plain form), the chemistry (ordered batched kernel, or one
-//    thread per cell), commit, validation - is one CUDA graph.  Every phase ORs its failure flags
+//    + update kernels of the plain form), the chemistry (ordered batched kernel, or the
+//    plain form), commit, validation - is one CUDA graph.  Every phase ORs its failure flags
 //    into one status block; the host reads it once per step.  Any flag discards the
 //    step and the host-controlled path below re-runs it.
 //  * host-controlled path: the ABI calls one by one with a status read after each,
@@ -191,7 +191,7 @@ cudaError_t enqueue_step(hf_stepper* st, double cfl, double* S0, double* T1, dou
     // commit, validate
     HF_Q(cudaMemsetAsync(&st->gst->counter, 0, 3 * sizeof(unsigned long long), s));  // work-queue heads
     if (st->chemistry) {
-        if (st->chem_form == HF_CHEM_PLAIN) {  // the drop-in form: one thread per cell
+        if (st->chem_form == HF_CHEM_PLAIN) {  // the drop-in form
             HF_Q(launch_chem(st->ns, HF_CHEM_PLAIN, X, P.comp_stride, st->cells, nc, 0.0, nullptr, st->rtol, st->atol,
                              st->trial, st->fail, st->gst, st->sm_count, s, nl, st->ddt));
         } else {

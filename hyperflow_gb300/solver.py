@@ -223,7 +223,8 @@ def euler_stage(ctx, level, u_in, u_out, h, first_order=False, u_old=None, form=
 def flux_adjoint(ctx, level, u_in, ubar_out, h, first_order=False):
     """Adjoint of one Euler stage (hf_flux_adjoint): u_in holds the forward stage's input
     with its ghosts filled, ubar_out the cotangent of the stage output (same layout);
-    returns a PatchArray holding J^T ubar_out on the interior cells."""
+    returns a PatchArray holding J^T ubar_out on the interior cells.  The branches are those
+    of the stage as a recorded run (FlowAdjoint) evaluates it."""
     out = u_in.like()
     ctx.check(ctx.lib.hf_flux_adjoint(ctx.h, ctypes.byref(level), ctypes.byref(u_in.patch), _ptr(u_in.data),
                                       _ptr(ubar_out.data), float(h), int(first_order), _ptr(out.data), _stream()),
@@ -263,10 +264,11 @@ class ConservativeInterp:
 class ChemistryBatch:
     """ChemistryBatch (src/chemistry_batch.hpp): all-or-nothing advance of a batch of cells.
 
-    form: "plain" (one thread per cell), "persistent" (device work queue; the same
-    per-cell step sequence as plain), or "batched" (persistent queue plus frozen-cell
-    screening, warm-started step sizes and a cost-ordered queue, using per-cell
-    history kept by this object between calls)."""
+    form: "plain" (one thread per cell), "persistent" (device work queue; bit for bit the
+    results of plain; both one cell per group of 8 lanes up to 64 cells per SM), or
+    "batched" (persistent queue plus frozen-cell screening, warm-started step sizes and a
+    cost-ordered queue, the costliest cells in groups, using per-cell history kept by this
+    object between calls; the first call has none and is slower)."""
 
     FORMS = {"plain": L.HF_CHEM_PLAIN, "persistent": L.HF_CHEM_PERSISTENT, "batched": -1}
 
@@ -493,7 +495,7 @@ class Stepper:
     """Strang-split reacting-Euler stepper on a uniform one-patch level.
 
     flux: "fused" or "plain"; chem: "batched" (work queue with per-cell history) or
-    "plain" (one thread per cell).
+    "plain" (ChemistryBatch's plain form).
 
     step(): flow(dt/2); react(dt); flow(dt/2) with rollback and dt halving
     (BlockAMR.cpp:409-419).  U0: (NV, ny, nx) float64 CUDA tensor."""

@@ -49,7 +49,8 @@ typedef enum hf_status {
 /* Boundary kinds: the strings of the reference's case JSON (BlockAMR.cpp:38-59). */
 enum { HF_BC_REFLECTING = 0, HF_BC_TRANSMISSIVE = 1, HF_BC_INFLOW = 2, HF_BC_WEDGE = 3 };
 
-/* Chemistry forms. */
+/* Chemistry forms.  Batches of up to 64 cells per SM run one cell per group of 8 lanes in both
+ * forms (the same step control, results to rounding as on one lane); larger ones as named. */
 enum { HF_CHEM_PLAIN = 0,      /* one thread per cell, one launch (the drop-in form) */
        HF_CHEM_PERSISTENT = 1  /* persistent launch pulling cells from a device work queue */ };
 
@@ -217,7 +218,11 @@ typedef struct hf_chem_history {
 /* Batched chemistry: the persistent work-queue kernel plus a frozen-cell screen (a cell whose
  * scaled derivative and Jacobian norms over dt are tiny takes one second-order Taylor step,
  * truncation error below 2e-5 tolerance units), warm-started step sizes and a cost-ordered
- * queue.  Same arguments, semantics and errors as hf_chem_advance (ChemistryBatch::advance,
+ * queue, the costliest cells one per group of 8 lanes.  A cell's result depends, to rounding,
+ * on whether it is among those, and so on the costs in history of the whole batch; the same
+ * batch with the same history gives the same bits.  Without a history (or with a new one) no
+ * cell's cost is known, none goes to a group, and the call waits for the longest chain on one
+ * lane.  Same arguments, semantics and errors as hf_chem_advance (ChemistryBatch::advance,
  * chemistry_batch.cpp:21-50); history may be NULL. */
 HF_EXPORT hf_status hf_chem_advance_batched(hf_ctx* ctx, double* U, int64_t comp_stride, const int64_t* cell_index,
                                             int64_t count, double dt, const double* dt_cell, double rtol,
@@ -288,6 +293,10 @@ HF_EXPORT void hf_flow_tape_destroy(hf_flow_tape* tape);
  * from a one-patch level's interior state U (ghosts filled from it by the boundary
  * conditions) to the stage output U - h div F of hf_flux_update (no Heun combination;
  * first_order as the forward stage took it), Ubar_in = J^T Ubar_out on the interior cells.
+ * The branches are those of the stage as hf_flow_record evaluates it, which agrees with
+ * hf_flux_update to rounding: where the contact speed at a face is zero to rounding (gas at
+ * rest, uniform pressure) the two may be on different sides of it, and the result is the
+ * one-sided derivative of the recorded stage's side.
  * U must hold the filled ghosts of the forward stage; U, Ubar_out and Ubar_in share the
  * patch layout (one domain-covering patch, ng = 2).  No wedge boundary.  HF_ERR_FACE if a
  * face state is inadmissible. */
@@ -301,7 +310,7 @@ HF_EXPORT hf_status hf_flux_adjoint(hf_ctx* ctx, const hf_level* level, const hf
  * budget is fixed up front and handed to its own pool (so a library allocation fails or
  * breaks the budget), or host code that must not take the device-wide synchronisation
  * that cudaMalloc and cudaFree can imply.  It needs no hf_ctx (hf_init allocates).  It
- * runs the plain form of hf_chem_advance (one thread per cell, same results, same
+ * runs the plain form of hf_chem_advance (same kernels and results, same
  * all-or-nothing semantics and error codes) with its scratch (trial states, failure
  * codes, status word) in one statically sized device array that every GPU loading this
  * library holds until the process exits: HF_NOALLOC_MAX_CELLS cells, about 1.8 MB.
@@ -470,7 +479,7 @@ HF_EXPORT hf_status hf_stepper_step(hf_stepper* st, double cfl, double* dt, void
  * and is re-run with host control (first-order redo, rollback, dt halving) exactly as
  * hf_stepper_step would.  Same results as nsteps calls of hf_stepper_step with *dt = 0.
  * *steps_done (may be NULL) receives the steps completed, also on error.  Either
- * chemistry form (batched, or plain: one thread per cell) runs inside the graphs. */
+ * chemistry form (batched or plain) runs inside the graphs. */
 HF_EXPORT hf_status hf_stepper_run(hf_stepper* st, int32_t nsteps, double cfl, int32_t* steps_done, void* stream);
 /* Copy the valid cells out, SoA [NV][ny][nx], to DEVICE memory. */
 HF_EXPORT hf_status hf_stepper_get(hf_stepper* st, double* U, void* stream);
