@@ -13,11 +13,14 @@
   cooperative setting whose queue stays empty on the sample can still engage, and cost,
   in later steps.  Otherwise the setting in force stays (unless it is more than MARGIN
   slower than the fastest): a sample that gains little from the library's own choice of
-  cells says nothing about the batches that gain 3 to 5 times from it.
+  cells says nothing about the batches that gain 3 to 5 times from it.  The other register
+  budgets are timed without groups: where a sample runs wholly in groups all budgets are
+  alike, and one of them would win by chance.
 * Stepper chemistry (tune_stepper): the same settings timed over a few whole graph
   steps of the caller's stepper from one start state, each candidate from a fresh
   stepper (its history builds up over the steps as it does in a run, so a cooperative
-  setting shows whether its queue engages and pays).  Small, tail-bound problems gain most
+  setting shows whether its queue engages and pays).  The setting in force stays unless one
+  is more than MARGIN faster.  Small, tail-bound problems gain most
   (a 1D detonation of 4,000 cells: 15.4 to 5.6 ms a step); the 2048 x 512 detonation's first
   steps gain 8%.
 * Flux form: one Euler stage of the workload's state with the plain per-face kernels and
@@ -36,24 +39,21 @@ from . import solver as S
 
 # the setting without groups, which the others are measured against; the library starts at (4, 17)
 CHEM_DEFAULT = (4, 16)
-CHEM_CANDIDATES = [CHEM_DEFAULT, (4, 17), (5, 17), (6, 17), (8, 17), (4, 3), (4, 5), (4, 7)]
+CHEM_CANDIDATES = [CHEM_DEFAULT, (4, 17), (5, 16), (6, 16), (8, 16), (4, 3), (4, 5), (4, 7)]
 MARGIN = 0.03
 STEP_CANDIDATES = [CHEM_DEFAULT, (4, 17), (4, 3), (4, 5), (4, 7)]
 
 
 def pick(sweep, key, default=CHEM_DEFAULT, margin=MARGIN, in_force=None):
-    """The sweep entry to apply: the fastest by `key` when it is more than `margin` faster
-    than the `default` setting's entry (or the sweep has no default entry); else the entry
-    of the setting `in_force`, when the sweep has one and the fastest is not more than
-    `margin` faster than it either; else the default's."""
+    """The sweep entry to apply: that of the setting `in_force` when the sweep has one and the
+    fastest by `key` is not more than `margin` faster; else likewise that of the `default`
+    setting; else the fastest."""
     best = min(sweep, key=lambda r: r[key])
-
-    def near(setting):
-        return [r for r in sweep if (r["blocks_per_sm"], r["coop_min_bucket"]) == tuple(setting or ()) and
-                best[key] >= (1.0 - margin) * r[key]]
-
-    base = near(default)
-    return (near(in_force) or base)[0] if base else best
+    for setting in (in_force, default):
+        for r in sweep:
+            if (r["blocks_per_sm"], r["coop_min_bucket"]) == setting and best[key] >= (1.0 - margin) * r[key]:
+                return r
+    return best
 
 
 def get_chem_tuning(ctx):
@@ -97,7 +97,9 @@ def tune_chemistry(ctx, X, dt, candidates=CHEM_CANDIDATES, apply=True):
             del field
     finally:
         set_chem_tuning(ctx, *before)
-    best = pick(sweep, "ms", in_force=before)
+    best = pick(sweep, "ms")
+    if (best["blocks_per_sm"], best["coop_min_bucket"]) == CHEM_DEFAULT:
+        best = pick(sweep, "ms", in_force=before)
     if apply:
         set_chem_tuning(ctx, best["blocks_per_sm"], best["coop_min_bucket"])
     return {"best": (best["blocks_per_sm"], best["coop_min_bucket"]), "sweep": sweep}

@@ -68,6 +68,7 @@ def run(ctx, which):
     ({(4, 17): 98.0}, (4, 17)),                           # it gains less than the margin
     ({(4, 17): 102.0}, (4, 17)),
     ({(4, 17): 60.0}, (4, 17)),
+    ({(4, 17): 102.0, (4, 7): 98.0}, (4, 16)),            # 4% behind the fastest, which is 2% ahead of no groups
     ({(4, 3): 60.0}, (4, 3)),                             # a clear winner
     ({(4, 17): 120.0}, (4, 16)),                          # the setting in force is a clear loser
 ])
@@ -77,11 +78,17 @@ def test_what_a_run_leaves(ctx, which, times, want):
     assert res["best"] == want == tune.get_chem_tuning(ctx)
 
 
+def test_settings_with_groups_that_are_alike(ctx):
+    """Whole steps: the setting in force stays; one call: the fastest of them is applied."""
+    ctx.times = {(4, 17): 60.0, (4, 5): 59.5}
+    assert run(ctx, "steps")["best"] == (4, 17) == tune.get_chem_tuning(ctx)
+    assert run(ctx, "call")["best"] == (4, 5)
+
+
 def test_a_setting_that_is_no_candidate_is_not_kept(ctx):
     ctx.now = [8, 11]
     assert run(ctx, "call")["best"] == tune.CHEM_DEFAULT
 
 
-def test_register_budgets_are_timed_with_the_rule_that_is_in_force():
-    assert all((b, 17) in tune.CHEM_CANDIDATES for b in (4, 5, 6, 8))
-    assert (4, 17) in tune.STEP_CANDIDATES
+def test_the_librarys_start_is_a_candidate():
+    assert (4, 17) in tune.CHEM_CANDIDATES and (4, 17) in tune.STEP_CANDIDATES
